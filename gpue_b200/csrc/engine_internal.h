@@ -22,6 +22,7 @@
 #include "ast.h"
 #include "aux_kernels.cuh"
 #include "registry.h"
+#include "stepper.cuh"
 
 namespace gpue_eng {
 
@@ -109,6 +110,15 @@ struct ZCfg {
     TSCounters ctr;
 };
 
+// The resident stepper of a 2D context (stepper.cuh): the kernel and its
+// cooperative grid, one CTA per C rows and C columns
+struct StepCfg {
+    const StepKernel* k = nullptr;
+    int threads = 0, blocks = 0;
+    size_t smem = 0;
+    int ready[2][2] = {};  // [tables][real time]: 1 the grid is resident at once, -1 it is not
+};
+
 struct GraphKey {
     int prec, gstate, parity, nsteps, scale_first, energy_last, guard, observables;
     bool operator<(const GraphKey& o) const {
@@ -149,6 +159,10 @@ struct gpue_ctx {
     gpue_eng::PlaneCfg plane[2];        // [precision]: XY-plane passes, if any
     gpue_eng::ZCfg zpass[2];            // [precision]: the TMA z pass, if any
     gpue_eng::XYCfg xy[2];              // [precision]: the cluster-free XY pass, if any
+    gpue_eng::StepCfg step[2];          // [precision]: the 2D resident stepper, if any
+    double2* step_slots = nullptr;      // the stepper's norm slots, zero between launches
+    bool line_plan = false;             // gpue_set_plan chose a line plan: steps run as line passes
+    std::map<gpue_eng::GraphKey, std::vector<gpue::StepPass>> step_seq;  // walks by segment shape
     bool have_wfc = false;
     bool pending_scale = false;  // scal[kScale] must multiply psi
     std::map<gpue_eng::GraphKey, gpue_eng::Segment> graphs;
@@ -192,7 +206,7 @@ enum {
     kNScal = 16
 };
 // counter slots: reductions in flight in one stream use distinct counters
-enum { kCtrNorm = 0, kCtrEkin = 1, kCtrEreal = 2, kCtrMisc = 3, kNCtr = 8 };
+enum { kCtrNorm = 0, kCtrEkin = 1, kCtrEreal = 2, kCtrMisc = 3, kCtrStep = 4, kNCtr = 8 };
 constexpr long kAuxPartials = 4096;  // partials reserved for the aux kernels
 
 // Records a message on the context and returns st.
@@ -281,6 +295,9 @@ gpue_status plan_zpass(gpue_ctx* c, int prec);
 // when planned it runs the plane passes of the step instead of the cluster
 // kernels.
 gpue_status plan_xy(gpue_ctx* c, int prec);
+// Plans the 2D resident stepper of precision prec (square grids whose tiles are
+// all resident at once); leaves it off otherwise.
+gpue_status plan_step(gpue_ctx* c, int prec);
 // The plane passes can run this context's steps now (no table or expression
 // fields, no in-plane gauge).
 bool plane_ok(const gpue_ctx* c, int prec);

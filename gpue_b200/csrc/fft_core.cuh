@@ -467,6 +467,37 @@ struct LineFFT {
         sync();
     }
 
+    // The same through alternating buffers: the next exchange writes the other
+    // one (sl and other swap), so its own barrier, which a thread only passes
+    // after this exchange's reads, separates them from the next write to this
+    // one and the trailing barrier goes.
+    template <int S, typename Sync>
+    static __device__ __forceinline__ void exchange2(cx<T> (&v)[E], int t, cx<T>*& sl,
+                                                     cx<T>*& other, Sync sync) {
+        constexpr int R = radix(S);
+        constexpr int Ns = ns_before(S);
+        constexpr int G = N / (R * P);
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const int j = t + P * q;
+            const int base = (j / Ns) * Ns * R + (j % Ns);
+#pragma unroll
+            for (int r = 0; r < R; ++r) sl[smem_phys(base + r * Ns)] = v[q * R + r];
+        }
+        sync();
+        constexpr int R2 = radix(S + 1);
+        constexpr int G2 = N / (R2 * P);
+#pragma unroll
+        for (int q = 0; q < G2; ++q) {
+            const int j = t + P * q;
+#pragma unroll
+            for (int r = 0; r < R2; ++r) v[q * R2 + r] = sl[smem_phys(j + r * (N / R2))];
+        }
+        cx<T>* const w = sl;
+        sl = other;
+        other = w;
+    }
+
     // One stage after the first: its twiddles are requested before the
     // exchange, so their latency overlaps the shared-memory round trip.
     template <int S, bool TWS, bool INV, typename Sync>
@@ -489,6 +520,27 @@ struct LineFFT {
         stage<1, TWS, INV>(v, t, sl, tw, sync);
         if constexpr (NS >= 3) stage<2, TWS, INV>(v, t, sl, tw, sync);
         if constexpr (NS >= 4) stage<3, TWS, INV>(v, t, sl, tw, sync);
+    }
+
+    template <int S, bool TWS, bool INV, typename Sync>
+    static __device__ __forceinline__ void stage2(cx<T> (&v)[E], int t, cx<T>*& sl,
+                                                  cx<T>*& other, const cx<T>* __restrict__ tw,
+                                                  Sync sync) {
+        StageTw<S, TWS> w;
+        w.load(t, tw);
+        exchange2<S - 1>(v, t, sl, other, sync);
+        compute<S, TWS, INV>(v, &w);
+    }
+
+    // forward with alternating exchange buffers (sl: the next one to write)
+    template <bool TWS = false, bool INV = false, typename Sync>
+    static __device__ __forceinline__ void forward2(cx<T> (&v)[E], int t, cx<T>*& sl,
+                                                    cx<T>*& other, const cx<T>* __restrict__ tw,
+                                                    Sync sync) {
+        compute<0, TWS, INV>(v, static_cast<const StageTw<0, TWS>*>(nullptr));
+        stage2<1, TWS, INV>(v, t, sl, other, tw, sync);
+        if constexpr (NS >= 3) stage2<2, TWS, INV>(v, t, sl, other, tw, sync);
+        if constexpr (NS >= 4) stage2<3, TWS, INV>(v, t, sl, other, tw, sync);
     }
 };
 

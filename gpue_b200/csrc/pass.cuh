@@ -222,6 +222,12 @@ __device__ __forceinline__ cx<T> apply(cx<T> v, cx<double> f) {
     }
 }
 
+// psi * f for a real f (the imaginary-time factors)
+template <typename T>
+__device__ __forceinline__ cx<T> apply_re(cx<T> v, double f) {
+    return cx<T>{(T)((double)v.x * f), (T)((double)v.y * f)};
+}
+
 template <typename T>
 __device__ __forceinline__ cx<double> unit_phase(double a);
 
@@ -297,7 +303,7 @@ __device__ __forceinline__ double decay(double a) {
 // no branch and the values' FP64 chains interleave.
 template <typename T, class L>
 __device__ __forceinline__ void op_vhalf_sep(cx<T> (&v)[L::E], int t, const double2* fa,
-                                             cx<double> lf, const PassArgs& a) {
+                                             cx<double> lf, const PassArgs& a, int gstate) {
     constexpr int E = L::E;
     bool small = true;
     if (a.gpe) {
@@ -312,12 +318,11 @@ __device__ __forceinline__ void op_vhalf_sep(cx<T> (&v)[L::E], int t, const doub
     if (!a.gpe) {
 #pragma unroll
         for (int e = 0; e < E; ++e) v[e] = apply(v[e], cmul(ld2(fa, L::index(t, e)), lf));
-    } else if (small && a.gstate == 0) {
+    } else if (small && gstate == 0) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const double gd = a.nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
-            const cx<double> f = cmul(ld2(fa, L::index(t, e)), lf);
-            v[e] = apply(v[e], cscale(f, taylor_decay(gd)));
+            v[e] = apply_re(v[e], fa[L::index(t, e)].x * lf.x * taylor_decay(gd));
         }
     } else if (small) {
 #pragma unroll
@@ -329,12 +334,26 @@ __device__ __forceinline__ void op_vhalf_sep(cx<T> (&v)[L::E], int t, const doub
     } else {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            cx<double> f = cmul(ld2(fa, L::index(t, e)), lf);
             const double gd = a.nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
-            if (a.gstate == 0) f = cscale(f, small_decay<T>(gd));
-            else f = cmul(f, small_phase<T>(gd));
-            v[e] = apply(v[e], f);
+            if (gstate == 0)
+                v[e] = apply_re(v[e], fa[L::index(t, e)].x * lf.x * small_decay<T>(gd));
+            else
+                v[e] = apply(v[e], cmul(cmul(ld2(fa, L::index(t, e)), lf), small_phase<T>(gd)));
         }
+    }
+}
+
+// OP_KPHASE, complex128: psi *= fa[k] * lf, lf the other axes' factors at the
+// line times the real scalings; real factors in imaginary time
+template <class L>
+__device__ __forceinline__ void op_kphase_f64(cx<double> (&v)[L::E], int t, const double2* fa,
+                                              cx<double> lf, int gstate) {
+    if (gstate == 0) {
+#pragma unroll
+        for (int e = 0; e < L::E; ++e) v[e] = cscale(v[e], fa[L::index(t, e)].x * lf.x);
+    } else {
+#pragma unroll
+        for (int e = 0; e < L::E; ++e) v[e] = cmul(v[e], cmul(ld2(fa, L::index(t, e)), lf));
     }
 }
 
@@ -414,7 +433,8 @@ __device__ __forceinline__ float nl_decay_delta64(double p) { return (float)expm
 // s^2 when a pending scale s is folded into dl instead of applied to v).
 template <class L>
 __device__ __forceinline__ void op_vhalf_f32(cx<float> (&v)[L::E], int t, const float2* dk,
-                                             float2 dl, const PassArgs& a, double nl64) {
+                                             float2 dl, const PassArgs& a, int gstate,
+                                             double nl64) {
     constexpr int E = L::E;
     const float nl = (float)nl64;
     bool small = true;
@@ -427,7 +447,7 @@ __device__ __forceinline__ void op_vhalf_f32(cx<float> (&v)[L::E], int t, const 
     if (!a.gpe) {
 #pragma unroll
         for (int e = 0; e < E; ++e) v[e] = dapply(v[e], dmul(dl, ldf2(dk, L::index(t, e))));
-    } else if (small && a.gstate == 0) {
+    } else if (small && gstate == 0) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const float dv = dl.x + ldf2(dk, L::index(t, e)).x +
@@ -447,7 +467,7 @@ __device__ __forceinline__ void op_vhalf_f32(cx<float> (&v)[L::E], int t, const 
         for (int e = 0; e < E; ++e) {
             const double p = nl64 * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
             const float2 dv = dmul(dl, ldf2(dk, L::index(t, e)));
-            const float2 dn = a.gstate == 0 ? float2{nl_decay_delta64(p), 0.f}
+            const float2 dn = gstate == 0 ? float2{nl_decay_delta64(p), 0.f}
                                             : nl_phase_delta64(p);
             v[e] = dapply(v[e], dmul(dv, dn));
         }
@@ -496,6 +516,97 @@ __device__ __forceinline__ void op_norm_f32(const cx<float> (&v)[E], KSum& acc) 
     acc.add((double)part);
 }
 
+// ------------------------------------------------------------- gauge factor --
+//
+// exp(-A p dt) / exp(-i A p dt) times gscale, with p = m dp, m the signed
+// frequency of index k (m = k - n for k >= n/2).  It is geometric in k: the
+// factor of k = t + P q + r n/RA is W^t A^q B^r, times W^-n for r >= RA/2
+// (t + P q < n/RA, so k >= n/2 exactly there), with W = w(dp), A = W^P,
+// B = W^(n/RA), all formed in FP64.  ang1 is the angle per unit m.
+
+struct GaugeConsts {
+    cx<double> wt, wa, wb, wn;  // W^t gscale, W^P, W^(n/RA), W^-n
+};
+
+template <class L>
+__device__ __forceinline__ GaugeConsts gauge_consts(int t, double ang1, int gstate,
+                                                    double gscale) {
+    constexpr int N = L::N, P = L::P, RA = L::radix(0);
+    if (gstate == 0)
+        return {{exp(-ang1 * t) * gscale, 0.0}, {exp(-ang1 * P), 0.0},
+                {exp(-ang1 * (N / RA)), 0.0}, {exp(ang1 * N), 0.0}};
+    return {cscale(unit_phase<double>(ang1 * t), gscale), unit_phase<double>(ang1 * P),
+            unit_phase<double>(ang1 * (N / RA)), unit_phase<double>(-ang1 * N)};
+}
+
+template <typename T, class L>
+__device__ __forceinline__ void op_gauge(cx<T> (&v)[L::E], const GaugeConsts& g, int gstate) {
+    constexpr int RA = L::radix(0), QN = L::E / RA;
+    static_assert(RA % 2 == 0, "the upper half of the spectrum starts at r = RA/2");
+    if (gstate == 0) {
+        double aq = g.wt.x;
+#pragma unroll
+        for (int q = 0; q < QN; ++q) {
+            double f = aq;
+#pragma unroll
+            for (int r = 0; r < RA; ++r) {
+                if (r == RA / 2) f *= g.wn.x;
+                v[q * RA + r] = apply_re(v[q * RA + r], f);
+                f *= g.wb.x;
+            }
+            aq *= g.wa.x;
+        }
+    } else {
+        cx<double> aq = g.wt;
+#pragma unroll
+        for (int q = 0; q < QN; ++q) {
+            cx<double> f = aq;
+#pragma unroll
+            for (int r = 0; r < RA; ++r) {
+                if (r == RA / 2) f = cmul(f, g.wn);
+                v[q * RA + r] = apply(v[q * RA + r], f);
+                f = cmul(f, g.wb);
+            }
+            aq = cmul(aq, g.wa);
+        }
+    }
+}
+
+// Complex64: the whole line's angles below 1/16, where the factor minus 1 comes
+// from its FP32 Taylor series (relative truncation below 2^-24) and is applied
+// as psi + d*psi, as the other complex64 factors are.  The FP64 chain costs a
+// conversion of every component each way, which run at a fraction of the FP32
+// rate: on the 1024^2 rotating case it was a third of the pass's issue slots.
+__device__ __forceinline__ bool gauge_small(double ang1, int n) {
+    return fabs(ang1) * (0.5 * n) < 0.0625;
+}
+template <class L>
+__device__ __forceinline__ void op_gauge_f32(cx<float> (&v)[L::E], int t, double ang1, int gstate,
+                                             double gscale) {
+    constexpr int N = L::N, RA = L::radix(0);
+    // the angle per unit m and the scale as hi + lo floats: the angle is then
+    // rounded once per element, and the rounded part of the scale (which would
+    // be a systematic error of every step) enters the factor
+    const float ch = (float)ang1, cl = (float)(ang1 - (double)ch), tf = (float)t;
+    const float s = (float)gscale;
+    const float eps = (float)((gscale - (double)s) * (double)N);  // gscale = 1/N
+#pragma unroll
+    for (int e = 0; e < L::E; ++e) {
+        const int r = e % RA;
+        const float m = tf + (float)(L::P * (e / RA) + r * (N / RA) - (r >= RA / 2 ? N : 0));
+        const float p = fmaf(m, ch, m * cl);
+        cx<float> w;
+        if (gstate == 0) {
+            w = dapply_re(v[e], nl_decay_delta(p) + eps);
+        } else {
+            float2 d = nl_phase_delta(p);
+            d.x += eps;
+            w = dapply(v[e], d);
+        }
+        v[e] = {w.x * s, w.y * s};
+    }
+}
+
 // ---------------------------------------------------------------- kernel --
 
 constexpr int kMaxPassThreads = 256;
@@ -530,11 +641,14 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
     using L = LineFFT<T, N, RA, RB, P, RC>;
     constexpr int E = L::E;
 
+    static_assert((P & (P - 1)) == 0, "threads per line are a power of two");
     const int C = blockDim.x / P;
     int c, t;
     if constexpr (STRIDED) {
         c = threadIdx.x % C;
-        t = threadIdx.x / C;
+        // (blockDim.x = C P: the mask changes nothing, but the known range lets
+        // the compiler fold the exchanges' padded offsets into constants)
+        t = (threadIdx.x / C) & (P - 1);
     } else {
         t = threadIdx.x % P;
         c = threadIdx.x / P;
@@ -642,9 +756,9 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     else if (a.axis == 1) lf = cmul(ld2(a.vfac[0], xi), ld2(a.vfac[2], zi));
                     else lf = cmul(ld2(a.vfac[0], xi), ld2(a.vfac[1], yi));
                     if constexpr (std::is_same<T, float>::value)
-                        op_vhalf_f32<L>(v, t, a.vd[a.axis], line_delta(lf), a, a.nl_coef);
+                        op_vhalf_f32<L>(v, t, a.vd[a.axis], line_delta(lf), a, a.gstate, a.nl_coef);
                     else
-                        op_vhalf_sep<T, L>(v, t, a.vfac[a.axis], lf, a);
+                        op_vhalf_sep<T, L>(v, t, a.vfac[a.axis], lf, a, a.gstate);
                     break;
                 }
                 case OP_KPHASE: {
@@ -676,11 +790,7 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     if constexpr (std::is_same<T, float>::value) {
                         op_kphase_f32<L>(v, t, a.kd[a.axis], line_delta(lf), (float)ks);
                     } else {
-                        lf = cscale(lf, ks);
-                        const double2* fa = a.kfac[a.axis];
-#pragma unroll
-                        for (int e = 0; e < E; ++e)
-                            v[e] = apply(v[e], cmul(ld2(fa, L::index(t, e)), lf));
+                        op_kphase_f64<L>(v, t, a.kfac[a.axis], cscale(lf, ks), a.gstate);
                     }
                     break;
                 }
@@ -712,52 +822,16 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                             break;
                         }
                     }
-                    // exp(-A p dt) / exp(-i A p dt) with p = m dp, m the signed
-                    // frequency of index k (m = k - n for k >= n/2): geometric in
-                    // k, so the factor of k = t + P q + r n/RA is
-                    // W^t A^q B^r (times W^-n above n/2) with W = w(dp),
-                    // A = W^P, B = W^(n/RA), formed in FP64.
                     const int src = a.gauge_src;
                     const int sidx = (src == 0) ? xi : (src == 1) ? yi : zi;
                     const double ang1 = a.gauge_coef * a.pos[src][sidx] * a.gauge_dt * a.dmom;
-                    constexpr int QN = E / RA;
-                    if (a.gstate == 0) {
-                        const double wt = exp(-ang1 * t) * a.gscale;
-                        const double wa = exp(-ang1 * P), wb = exp(-ang1 * (N / RA));
-                        const double wn = exp(ang1 * N);
-                        double aq = wt;
-#pragma unroll
-                        for (int q = 0; q < QN; ++q) {
-                            double f = aq;
-#pragma unroll
-                            for (int r = 0; r < RA; ++r) {
-                                const int e = q * RA + r;
-                                const double ff = (t + P * q + r * (N / RA) >= N / 2) ? f * wn : f;
-                                v[e] = apply(v[e], cx<double>{ff, 0.0});
-                                f *= wb;
-                            }
-                            aq *= wa;
-                        }
-                    } else {
-                        cx<double> wt = cscale(unit_phase<double>(ang1 * t), a.gscale);
-                        const cx<double> wa = unit_phase<double>(ang1 * P);
-                        const cx<double> wb = unit_phase<double>(ang1 * (N / RA));
-                        const cx<double> wn = unit_phase<double>(-ang1 * N);
-                        cx<double> aq = wt;
-#pragma unroll
-                        for (int q = 0; q < QN; ++q) {
-                            cx<double> f = aq;
-#pragma unroll
-                            for (int r = 0; r < RA; ++r) {
-                                const int e = q * RA + r;
-                                const cx<double> ff =
-                                    (t + P * q + r * (N / RA) >= N / 2) ? cmul(f, wn) : f;
-                                v[e] = apply(v[e], ff);
-                                f = cmul(f, wb);
-                            }
-                            aq = cmul(aq, wa);
+                    if constexpr (std::is_same<T, float>::value) {
+                        if (gauge_small(ang1, N)) {
+                            op_gauge_f32<L>(v, t, ang1, a.gstate, a.gscale);
+                            break;
                         }
                     }
+                    op_gauge<T, L>(v, gauge_consts<L>(t, ang1, a.gstate, a.gscale), a.gstate);
                     break;
                 }
                 case OP_NORM:

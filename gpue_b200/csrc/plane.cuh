@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(PlaneShape<T, N, RA, RB, P, RC, LPR_>::THREADS
                     cscale(cmul(ld2(a.vfac[1], y), ld2(a.vfac[2], (int)z)), sc);
                 // the pending scale is folded into the factor, so the density
                 // of the unscaled values takes it squared
-                op_vhalf_f32<L>(v, rt, dx_s, line_delta(lf), a, a.nl_coef * sc * sc);
+                op_vhalf_f32<L>(v, rt, dx_s, line_delta(lf), a, a.gstate, a.nl_coef * sc * sc);
                 L::template forward<true>(v, rt, srow, twp, row_sync);
             } else {
 #pragma unroll
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(PlaneShape<T, N, RA, RB, P, RC, LPR_>::THREADS
 #pragma unroll
                 for (int e = 0; e < E; ++e) v[e].y = -v[e].y;
                 const cx<double> lf = cmul(ld2(a.vfac[0], x_col), ld2(a.vfac[2], (int)z));
-                op_vhalf_f32<L>(v, ct, dy_s, line_delta(lf), a, a.nl_coef);
+                op_vhalf_f32<L>(v, ct, dy_s, line_delta(lf), a, a.gstate, a.nl_coef);
                 if (a.red.kind == RED_NORM) op_norm_f32<E>(v, acc);
             }
             cx<T>* o = out + (size_t)z * plane + x_col;

@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
                         cscale(cmul(ld2(a.vfac[1], y), ld2(a.vfac[2], z)), sc);
                     // the pending scale is folded into the factor, so the
                     // density of the unscaled values takes it squared
-                    op_vhalf_f32<L>(v, t, d0_s, line_delta(lf), a, a.nl_coef * sc * sc);
+                    op_vhalf_f32<L>(v, t, d0_s, line_delta(lf), a, a.gstate, a.nl_coef * sc * sc);
                 }
                 L::template forward<true>(v, t, sl, twp, sync);
             } else if constexpr (KIND == TS_XY_INV) {
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
                 if (!rows) {
                     const int x = tile * LT + l;
                     const cx<double> lf = cmul(ld2(a.vfac[0], x), ld2(a.vfac[2], z));
-                    op_vhalf_f32<L>(v, t, d1_s, line_delta(lf), a, a.nl_coef);
+                    op_vhalf_f32<L>(v, t, d1_s, line_delta(lf), a, a.gstate, a.nl_coef);
                     if (a.red.kind == RED_NORM) op_norm_f32<E>(v, acc);
                 }
             } else {
