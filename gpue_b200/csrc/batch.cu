@@ -88,15 +88,72 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
            c->xy[prec].k && c->zpass[prec].k && plane_ok(c, prec);
 }
 
+// Cluster sizes of a run's 2D solves (0: not on the cluster stepper).  A solve
+// starts at the smallest cluster that holds its field; while the device has
+// room, the one with most points per CTA doubles, so a mix finishes together
+// and few solves still use the device.  A cluster must lie in one GPC, so the
+// device holds fewer large ones than its SMs suggest (7 of 16 CTAs, not 9):
+// each counts as the share of the device that the occupancy query says.  16
+// solves of 256^2 complex64 as clusters of 8 take two waves, 52 us a step; as
+// clusters of 4, one.  Results do not depend on the choice.
+std::vector<int> cluster_sizes(const BatchRun& r) {
+    const size_t n = r.ctx.size();
+    std::vector<int> cs(n, 0);
+    const char* env = std::getenv("GPUE_BATCH_MEGA");
+    if (env && env[0] == '0') return cs;
+    auto share = [&](size_t i, int s) {  // of the device; > 1: such a cluster does not fit
+        const ClusterKernel* k = r.ctx[i]->cluster[r.ctx[i]->prec].k;
+        const int m = clusters_resident(k, k->many[r.gstate], s);
+        return m > 0 ? 1.0 / m : 2.0;
+    };
+    double total = 0;
+    for (size_t i = 0; i < n; ++i) {
+        gpue_ctx* c = r.ctx[i];
+        const ClusterKernel* k = c->cluster[c->prec].k;
+        if (!k || c->ext || c->time_dep || c->line_plan) continue;
+        int max_smem = 0;
+        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+        int s = 1;
+        while (s < c->cluster[c->prec].cs && k->smem(s) > (size_t)max_smem) s *= 2;
+        if (k->smem(s) > (size_t)max_smem || share(i, s) > 1.0) continue;
+        cs[i] = s;
+        total += share(i, s);
+    }
+    std::vector<char> full(n, 0);
+    for (;;) {
+        int best = -1;
+        double most = 0;
+        for (size_t i = 0; i < n; ++i) {
+            const double load = cs[i] ? (double)r.ctx[i]->N / cs[i] : 0.0;
+            if (!full[i] && load > most) {
+                most = load;
+                best = (int)i;
+            }
+        }
+        if (best < 0) break;
+        const int s = 2 * cs[best];
+        if (s > r.ctx[best]->cluster[r.ctx[best]->prec].cs ||
+            total + share(best, s) - share(best, cs[best]) > 1.0) {
+            full[best] = 1;
+            continue;
+        }
+        total += share(best, s) - share(best, cs[best]);
+        cs[best] = s;
+    }
+    return cs;
+}
+
 void group_solves(BatchRun& r, int probe) {
     r.groups.clear();
     std::map<std::string, int> by_sig;
+    const std::vector<int> cs = cluster_sizes(r);
     for (size_t i = 0; i < r.ctx.size(); ++i) {
         gpue_ctx* c = r.ctx[i];
         const int off = r.offset[i];
         const bool tile = tile_eligible(c, c->prec);
         const std::string sig =
             std::to_string((int)r.guard[i]) + "/" + (tile ? "tile/" : "") +
+            (cs[i] ? "cluster" + std::to_string(cs[i]) + "/" : "") +
             pass_signature(c, c->prec,
                            solve_passes(c, off, off + probe, r.gstate, r.guard[i], r.scale_step0,
                                         tile));
@@ -107,7 +164,8 @@ void group_solves(BatchRun& r, int probe) {
             g.prec = c->prec;
             g.guard = r.guard[i];
             g.tile = tile;
-            g.mega = !tile && mega_eligible(c, c->prec);
+            g.cluster = cs[i];
+            g.mega = !tile && !g.cluster && mega_eligible(c, c->prec);
             r.groups.push_back(g);
         }
         r.groups[it->second].members.push_back((int)i);
@@ -247,6 +305,51 @@ gpue_status plan_mega(const BatchRun& r, int prec, int s0, int s1, ArgSink& sink
     return GPUE_OK;
 }
 
+// The steps [s0, s1) of a cluster group as one launch, one cluster per solve.
+static gpue_status plan_cluster_launch(const BatchRun& r, const BGroup& g, int s0, int s1,
+                                       ArgSink& sink, std::vector<LaunchOp>& ops,
+                                       std::string& err) {
+    const int n = (int)g.members.size();
+    std::vector<ClusterArgs> args(n);
+    for (int k = 0; k < n; ++k) {
+        const int m = g.members[k];
+        gpue_ctx* c = r.ctx[m];
+        ClusterArgs& a = args[k];
+        std::memset(&a, 0, sizeof a);  // equal arrays are stored once: no stray bytes
+        gpue_status st = stepper_consts(c, g.prec, r.gstate, a.a, a.gauge_ang);
+        if (st) {
+            err = c->err;
+            return st;
+        }
+        a.scal_norm = c->scal + kScale;
+        a.scal_guard = c->scal + kGuard;
+        a.target_norm = c->scal + kTargetImag;
+        a.target_guard = c->scal + kTargetReal;
+        const int i0 = r.offset[m] + s0;
+        const std::vector<StepPass> walk =
+            step_walk(c, i0, s1 - s0, r.gstate, r.gstate == 0 && (i0 > 0 || r.scale_step0),
+                      r.guard[m] ? 1 : 0);
+        const void* dseq = nullptr;
+        st = sink.put(walk.data(), walk.size() * sizeof(StepPass), &dseq, err);
+        if (st) return st;
+        a.seq = static_cast<const StepPass*>(dseq);
+        a.nseq = (int)walk.size();
+    }
+    const void* dargs = nullptr;
+    gpue_status st = sink.put(args.data(), args.size() * sizeof(ClusterArgs), &dargs, err);
+    if (st) return st;
+    gpue_ctx* c0 = r.ctx[g.members[0]];
+    const ClusterKernel* k = c0->cluster[g.prec].k;
+    const void* fn = k->many[r.gstate];
+    const int cs = g.cluster;
+    ops.push_back([=](cudaStream_t s) {
+        const ClusterArgs* p = static_cast<const ClusterArgs*>(dargs);
+        void* params[] = {&p};
+        launch_cluster(k, fn, cs, n, s, params);
+    });
+    return GPUE_OK;
+}
+
 gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink& sink,
                          SegPlan& sp, std::string& err) {
     sp.lanes.assign(r.groups.size(), {});
@@ -265,10 +368,16 @@ gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink&
         const int n = (int)g.members.size();
         gpue_ctx* c0 = r.ctx[g.members[0]];
         std::vector<std::vector<LPass>> lists(n);
+        if (g.cluster) {
+            gpue_status st = plan_cluster_launch(r, g, s0, s1, sink, out_ops, err);
+            if (st) return st;
+            sp.launches++;
+            if (!check) continue;
+        }
         for (int k = 0; k < n; ++k) {
             const int m = g.members[k];
             gpue_ctx* c = r.ctx[m];
-            if (!g.mega)
+            if (!g.mega && !g.cluster)
                 lists[k] = solve_passes(c, r.offset[m] + s0, r.offset[m] + s1, r.gstate,
                                         r.guard[m], r.scale_step0, g.tile);
             if (check)
@@ -327,7 +436,8 @@ gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink&
             const unsigned grid = (unsigned)(n * lc.ntiles);
             const unsigned threads = (unsigned)lc.threads;
             const size_t smem = lc.smem;
-            const bool pdl = j > 0;  // follows a pass kernel on this lane
+            // follows a pass kernel on this lane (a cluster launch is none)
+            const bool pdl = j > 0;
             out_ops.push_back([=](cudaStream_t s) {
                 launch_kernel(fn, grid, threads, smem, s, pdl,
                               static_cast<const PassArgs*>(dargs),
@@ -696,7 +806,7 @@ gpue_status gpue_batch_evolve(gpue_batch* b, int32_t gstate, const gpue_batch_op
         std::snprintf(tb, sizeof tb, "%a:", run.thr);
         k += tb;
         for (const BGroup& g : run.groups) {
-            k += "{" + std::to_string(g.guard) + "/" +
+            k += "{" + std::to_string(g.guard) + "/" + std::to_string(g.cluster) + "/" +
                  pass_signature(run.ctx[g.members[0]], g.prec,
                                 solve_passes(run.ctx[g.members[0]], 0, 3, gstate, g.guard,
                                              false, g.tile)) + "}";

@@ -33,6 +33,7 @@ struct BGroup {
     int prec = 0;
     bool guard = false;
     bool mega = false;         // its solves run on the persistent multi-size kernel
+    int cluster = 0;           // > 0: each solve runs on a cluster of that many CTAs
     bool tile = false;         // 3D complex64: the three tile-stream passes per step, per solve
     std::vector<int> members;  // indices into BatchRun::ctx
 };

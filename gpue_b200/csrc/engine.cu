@@ -985,12 +985,6 @@ gpue_status enqueue_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, boo
     return GPUE_OK;
 }
 
-// The steps of a segment can run as one resident launch: no per-step arguments
-// (ramp, expressions) and no line plan asked for.
-bool step_ok(gpue_ctx* c, int prec, int gstate) {
-    return c->step[prec].k && !c->time_dep && !c->line_plan && step_ready(c, prec, gstate);
-}
-
 // Most steps one resident launch holds (at most 6 passes a step)
 constexpr int kStepChunk = kStepMaxSeq / 6;
 
@@ -1027,6 +1021,8 @@ bool same_walk(const StepPass* a, const StepPass* b, size_t n) {
     return n == 0 || std::memcmp(a, b, n * sizeof(StepPass)) == 0;
 }
 
+}  // namespace
+
 // The same for any n: the pattern repeats every 4 steps (gauge order i % 2,
 // guard period 1, 2 or 4), so a long walk is a short one with its middle
 // repeated, checked on the next longer one.
@@ -1046,12 +1042,116 @@ std::vector<StepPass> step_walk(gpue_ctx* c, int i0, int n, int gstate, bool sca
     return out;
 }
 
-}  // namespace
+gpue_status stepper_consts(gpue_ctx* c, int prec, int gstate, PassArgs& a, double (&ang)[2]) {
+    LPass lp;
+    lp.gauge_dt = gstate == 0 ? c->p.gdt : c->p.dt;
+    gpue_status st = make_pass_args(c, prec, lp, gstate, a);
+    if (st) return st;
+    double axc, ayc;
+    gauge_coefs(c, axc, ayc);
+    const bool gauge = c->p.corotating && !c->use_atab;
+    ang[0] = gauge && axis_gauge_active(c, 0) ? axc * lp.gauge_dt * a.dmom : 0.0;
+    ang[1] = gauge && axis_gauge_active(c, 1) ? ayc * lp.gauge_dt * a.dmom : 0.0;
+    return GPUE_OK;
+}
 
-// Steps [i0, i1) as one cooperative launch.
+cudaError_t launch_cluster(const ClusterKernel* k, const void* fn, int cs, int clusters,
+                           cudaStream_t s, void** args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * cs);
+    cfg.blockDim = dim3(k->threads);
+    cfg.dynamicSmemBytes = k->smem(cs);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+int clusters_resident(const ClusterKernel* k, const void* fn, int cs) {
+    // asked once per kernel and size: the answer is the device's and does not
+    // change (every device of a node is of one kind)
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, int> known;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find({fn, cs});
+    if (it != known.end()) return it->second;
+    const int smem = (int)k->smem(cs);
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(k->threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    // (the attribute keeps the largest size asked for: smaller clusters of a
+    // length need more shared memory)
+    cudaFuncAttributes fa;
+    const bool ok =
+        cudaFuncGetAttributes(&fa, fn) == cudaSuccess &&
+        (fa.maxDynamicSharedSizeBytes >= smem ||
+         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+             cudaSuccess) &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();  // not an error of the call that asks
+        n = 0;
+    }
+    known[{fn, cs}] = n;
+    return n;
+}
+
+gpue_status plan_cluster(gpue_ctx* c, int prec) {
+    ClusterCfg& cc = c->cluster[prec];
+    cc = ClusterCfg();
+    if (c->dim != 2) return GPUE_OK;
+    const int n = c->ax[0].n;
+    const ClusterKernel* k = find_cluster_kernel(kprec(prec), n);
+    if (!k) return GPUE_OK;
+    int max_smem = 0;
+    CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    int cs = kClusterMax;
+    while (cs > 1 && n / cs < 4) cs /= 2;
+    if (k->smem(cs) > (size_t)max_smem) return GPUE_OK;
+    cc.k = k;
+    cc.cs = cs;
+    return GPUE_OK;
+}
+
+// Whether a solve stepped alone takes the cluster stepper: up to 64^2, where
+// its cheaper barriers outweigh its 16 SMs (complex128 per step as a cluster
+// and as a grid: 16^2 4.8 and 6.0 us, 64^2 6.5 and 7.3, 128^2 9.5 and 8.9).
+constexpr int kClusterAlone = 64;
+static bool cluster_ok(gpue_ctx* c, int prec, int gstate) {
+    ClusterCfg& cc = c->cluster[prec];
+    if (!cc.k || c->ext) return false;
+    if (c->ax[0].n > kClusterAlone) return false;
+    int& r = cc.ready[gstate ? 1 : 0];
+    if (r == 0) r = clusters_resident(cc.k, cc.k->one[gstate ? 1 : 0], cc.cs) > 0 ? 1 : -1;
+    return r > 0;
+}
+
+// The steps of a segment can run as one resident launch: no per-step arguments
+// (ramp, expressions) and no line plan asked for.
+bool step_ok(gpue_ctx* c, int prec, int gstate) {
+    if (!c->step[prec].k || c->time_dep || c->line_plan) return false;
+    return cluster_ok(c, prec, gstate) || step_ready(c, prec, gstate);
+}
+
+// Steps [i0, i1) as one launch: a cluster, or a cooperative grid.
 gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool scale_first,
                          int guard) {
-    const StepCfg& sc = c->step[prec];
     const GraphKey key{prec, gstate, i0 % 4, i1 - i0, scale_first ? 1 : 0, 0, guard, 0};
     auto it = c->step_seq.find(key);
     if (it == c->step_seq.end())
@@ -1060,15 +1160,8 @@ gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool
     if (walk.size() > (size_t)kStepMaxSeq)
         return fail(c, GPUE_ERR_STATE, "a resident launch holds at most %d passes", kStepMaxSeq);
     StepArgs s;
-    LPass lp;
-    lp.gauge_dt = gstate == 0 ? c->p.gdt : c->p.dt;
-    gpue_status st = make_pass_args(c, prec, lp, gstate, s.a);
+    gpue_status st = stepper_consts(c, prec, gstate, s.a, s.gauge_ang);
     if (st) return st;
-    double axc, ayc;
-    gauge_coefs(c, axc, ayc);
-    const bool gauge = c->p.corotating && !c->use_atab;
-    s.gauge_ang[0] = gauge && axis_gauge_active(c, 0) ? axc * lp.gauge_dt * s.a.dmom : 0.0;
-    s.gauge_ang[1] = gauge && axis_gauge_active(c, 1) ? ayc * lp.gauge_dt * s.a.dmom : 0.0;
     s.sync = c->counters + kCtrStep;
     s.slots = c->step_slots;
     s.scal_norm = c->scal + kScale;
@@ -1078,6 +1171,14 @@ gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool
     s.err = c->dflags + 3;
     s.nseq = (int)walk.size();
     std::copy(walk.begin(), walk.end(), s.seq);
+    void* args[] = {&s};
+    const ClusterCfg& cc = c->cluster[prec];
+    if (cluster_ok(c, prec, gstate)) {
+        CK(launch_cluster(cc.k, cc.k->one[gstate ? 1 : 0], cc.cs, 1, c->stream, args));
+        c->launches++;
+        return GPUE_OK;
+    }
+    const StepCfg& sc = c->step[prec];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sc.blocks);
     cfg.blockDim = dim3(sc.threads);
@@ -1088,7 +1189,6 @@ gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    void* args[] = {&s};
     CK(cudaLaunchKernelExC(&cfg, sc.k->fn[c->ext ? 1 : 0][gstate ? 1 : 0], args));
     c->launches++;
     return GPUE_OK;
@@ -1523,6 +1623,7 @@ gpue_status gpue_ctx_create(const gpue_params* p, gpue_ctx** out) {
     if (!st) st = plan_zpass(c, c->prec);
     if (!st) st = plan_xy(c, c->prec);
     if (!st) st = plan_step(c, c->prec);
+    if (!st) st = plan_cluster(c, c->prec);
     if (st) return st;
     const char* tune = std::getenv("GPUE_AUTOTUNE");
     if (tune && tune[0] == '1') {
@@ -2135,6 +2236,14 @@ int find_pass_kernels(int prec, int n, const PassKernel** out, int cap) {
 const StepKernel* find_step_kernel(int prec, int n) {
     int cnt = 0;
     const StepKernel* t = prec == PREC_F32 ? step_table_f32(&cnt) : step_table_f64(&cnt);
+    for (int i = 0; i < cnt; ++i)
+        if (t[i].n == n) return &t[i];
+    return nullptr;
+}
+
+const ClusterKernel* find_cluster_kernel(int prec, int n) {
+    int cnt = 0;
+    const ClusterKernel* t = prec == PREC_F32 ? cluster_table_f32(&cnt) : cluster_table_f64(&cnt);
     for (int i = 0; i < cnt; ++i)
         if (t[i].n == n) return &t[i];
     return nullptr;

@@ -23,6 +23,7 @@
 #include "aux_kernels.cuh"
 #include "registry.h"
 #include "stepper.cuh"
+#include "cluster_step.cuh"
 
 namespace gpue_eng {
 
@@ -119,6 +120,13 @@ struct StepCfg {
     int ready[2][2] = {};  // [tables][real time]: 1 the grid is resident at once, -1 it is not
 };
 
+// The cluster-resident stepper of a 2D context (cluster_step.cuh)
+struct ClusterCfg {
+    const ClusterKernel* k = nullptr;
+    int cs = 0;            // CTAs per cluster of a solve stepped alone
+    int ready[2] = {};     // [real time]: 1 such a cluster fits the device, -1 it does not
+};
+
 struct GraphKey {
     int prec, gstate, parity, nsteps, scale_first, energy_last, guard, observables;
     bool operator<(const GraphKey& o) const {
@@ -160,6 +168,7 @@ struct gpue_ctx {
     gpue_eng::ZCfg zpass[2];            // [precision]: the TMA z pass, if any
     gpue_eng::XYCfg xy[2];              // [precision]: the cluster-free XY pass, if any
     gpue_eng::StepCfg step[2];          // [precision]: the 2D resident stepper, if any
+    gpue_eng::ClusterCfg cluster[2];    // [precision]: the 2D cluster stepper, if any
     double2* step_slots = nullptr;      // the stepper's norm slots, zero between launches
     bool line_plan = false;             // gpue_set_plan chose a line plan: steps run as line passes
     std::map<gpue_eng::GraphKey, std::vector<gpue::StepPass>> step_seq;  // walks by segment shape
@@ -298,6 +307,22 @@ gpue_status plan_xy(gpue_ctx* c, int prec);
 // Plans the 2D resident stepper of precision prec (square grids whose tiles are
 // all resident at once); leaves it off otherwise.
 gpue_status plan_step(gpue_ctx* c, int prec);
+// Plans the 2D cluster stepper of precision prec (lengths whose field fits a
+// cluster's shared memory); leaves it off otherwise.
+gpue_status plan_cluster(gpue_ctx* c, int prec);
+// How many clusters of cs CTAs of kernel fn the device holds at once (0: none
+// fits); prepares fn for its launches.  Asked before a kernel's first launch,
+// so only kernels in use are loaded.
+int clusters_resident(const ClusterKernel* k, const void* fn, int cs);
+// Launches `clusters` clusters of cs CTAs.
+cudaError_t launch_cluster(const ClusterKernel* k, const void* fn, int cs, int clusters,
+                           cudaStream_t s, void** args);
+// The walk of a context's steps [i0, i0 + n) (stepper.cuh).
+std::vector<StepPass> step_walk(gpue_ctx* c, int i0, int n, int gstate, bool scale_first,
+                                int guard);
+// The rotation gauge's angles per momentum index and unit position, and the
+// per-call constants of a stepper launch.
+gpue_status stepper_consts(gpue_ctx* c, int prec, int gstate, PassArgs& a, double (&ang)[2]);
 // The plane passes can run this context's steps now (no table or expression
 // fields, no in-plane gauge).
 bool plane_ok(const gpue_ctx* c, int prec);
