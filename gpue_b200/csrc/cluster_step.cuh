@@ -236,7 +236,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
                         if constexpr (std::is_same<T, float>::value)
                             op_vhalf_f32<L>(v, t, vx_s, line_delta(lf), a, gstate, a.nl_coef);
                         else
-                            op_vhalf_sep<T, L>(v, t, vx_s, lf, a, gstate);
+                            op_vhalf_sep<T, L>(v, t, vx_s, lf, a, gstate, a.nl_coef);
                         break;
                     }
                     case OP_KPHASE: {

@@ -390,7 +390,8 @@ gpue_status plan_zpass(gpue_ctx* c, int prec) {
     zc.k = nullptr;
     const char* env = std::getenv("GPUE_ZTMA");
     if (env && env[0] == '0') return GPUE_OK;
-    if (c->dim != 3 || c->ax[0].n % 16 || c->ax[2].n > 256) return GPUE_OK;
+    const int per = (int)(elem_size(prec) / 8), lt = 16 / per;  // 8-byte elements per value, lines per tile
+    if (c->dim != 3 || c->ax[0].n % lt || c->ax[2].n > 256) return GPUE_OK;
     const ZPassKernel* k = find_zpass_kernel(kprec(prec), c->ax[2].n);
     EncodeTiled enc = encode_tiled();
     if (!k || !enc) return GPUE_OK;
@@ -401,13 +402,13 @@ gpue_status plan_zpass(gpue_ctx* c, int prec) {
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k->fn, k->threads, k->smem));
     if (per_sm < 1) return GPUE_OK;
-    // the field as nx x ny x nz elements of 8 bytes (one complex64 each); a
-    // box is 16 x-columns of one y-row over all planes, landed with the
-    // 128-byte swizzle (its rows are 16 x 8 = 128 bytes)
-    const cuuint64_t dims[3] = {(cuuint64_t)c->ax[0].n, (cuuint64_t)c->ax[1].n,
+    // the field as elements of 8 bytes (one complex64, half a complex128); a box
+    // is 128 bytes of x-columns of one y-row over all planes, landed with the
+    // 128-byte swizzle
+    const cuuint64_t dims[3] = {(cuuint64_t)c->ax[0].n * per, (cuuint64_t)c->ax[1].n,
                                 (cuuint64_t)c->ax[2].n};
-    const cuuint64_t strides[2] = {(cuuint64_t)c->ax[0].n * 8,
-                                   (cuuint64_t)c->ax[0].n * c->ax[1].n * 8};
+    const cuuint64_t strides[2] = {(cuuint64_t)c->ax[0].n * per * 8,
+                                   (cuuint64_t)c->ax[0].n * c->ax[1].n * per * 8};
     const cuuint32_t box[3] = {16, 1, (cuuint32_t)c->ax[2].n};
     const cuuint32_t estr[3] = {1, 1, 1};
     if (enc(&zc.tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, state_of(c, prec), dims, strides, box,
@@ -416,11 +417,21 @@ gpue_status plan_zpass(gpue_ctx* c, int prec) {
         return GPUE_OK;
     gpue_status st = alloc_counters(c, zc.ctr);
     if (st) return st;
-    const long tiles = (long)(c->ax[0].n / 16) * c->ax[1].n;
+    const long tiles = (long)(c->ax[0].n / lt) * c->ax[1].n;
     zc.blocks = (int)std::min<long>((long)per_sm * c->sms, tiles);
     zc.k = k;
     return GPUE_OK;
 }
+
+// Least points for the tile passes in complex128, and in either precision with
+// the rotation gauge (4 launches a step instead of 7 line passes).  An XY launch
+// has two dependent tile phases, about 9 us of latency that smaller fields,
+// which lie in L2 anyway, do not earn back.  Per step on B200, line passes and
+// tile passes: complex128 96^3 52 and 65 us, 128^3 125 and 87; with the gauge
+// complex128 96^3 85 and 85, 128^3 180 and 145, complex64 128^3 102 and 102,
+// 192^3 294 and 260.
+constexpr long kTileMin64 = 1L << 20;
+constexpr long kTileGaugeMin32 = 1L << 22;
 
 gpue_status plan_xy(gpue_ctx* c, int prec) {
     XYCfg& xc = c->xy[prec];
@@ -428,26 +439,32 @@ gpue_status plan_xy(gpue_ctx* c, int prec) {
     const char* env = std::getenv("GPUE_XY");
     if (env && env[0] == '0') return GPUE_OK;
     if (c->dim != 3 || c->ax[0].n != c->ax[1].n || c->ax[0].n > 256) return GPUE_OK;
+    if (prec == GPUE_PREC_FP64 && c->N < kTileMin64) return GPUE_OK;
     const XYKernel* k = find_xy_kernel(kprec(prec), c->ax[0].n);
     EncodeTiled enc = encode_tiled();
     if (!k || !enc) return GPUE_OK;
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     if (k->smem > max_smem) return GPUE_OK;
+    const int n = c->ax[0].n;
+    const int per = (int)(elem_size(prec) / 8), lt = 16 / per;  // 8-byte elements per value, lines per tile
+    const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
     int per_sm = 1 << 30;
-    for (const void* fn : {k->fwd, k->inv}) {
+    for (const void* fn : {k->fwd, gauge ? k->inv_gy : k->inv, gauge ? k->inv_gx : k->inv}) {
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
-        int n = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, k->threads, k->smem));
-        per_sm = std::min(per_sm, n);
+        int b = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, k->threads, k->smem));
+        per_sm = std::min(per_sm, b);
     }
     if (per_sm < 1) return GPUE_OK;
-    const int n = c->ax[0].n;
-    const cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)c->ax[2].n};
-    const cuuint64_t strides[2] = {(cuuint64_t)n * 8, (cuuint64_t)n * n * 8};
-    // x-tiles: 16 whole rows, as they lie; y-tiles: 16 x-columns over all
-    // y, landed with the 128-byte swizzle (rows of 16 x 8 = 128 bytes)
-    const cuuint32_t boxx[3] = {(cuuint32_t)n, 16, 1}, boxy[3] = {16, (cuuint32_t)n, 1};
+    xc.gauge = gauge;
+    const cuuint64_t dims[3] = {(cuuint64_t)n * per, (cuuint64_t)n, (cuuint64_t)c->ax[2].n};
+    const cuuint64_t strides[2] = {(cuuint64_t)n * per * 8, (cuuint64_t)n * n * per * 8};
+    // complex64 x-tiles: 16 whole rows, as they lie (complex128 ones are copied
+    // without a map); y-tiles: 128 bytes of x-columns over all y, landed with
+    // the 128-byte swizzle
+    const cuuint32_t boxx[3] = {(cuuint32_t)std::min(n, 256), 16, 1},
+                     boxy[3] = {16, (cuuint32_t)n, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     for (int w = 0; w < 2; ++w)
         if (enc(w ? &xc.tmy : &xc.tmx, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, state_of(c, prec),
@@ -458,9 +475,19 @@ gpue_status plan_xy(gpue_ctx* c, int prec) {
             return GPUE_OK;
     gpue_status st = alloc_counters(c, xc.ctr);
     if (st) return st;
+    // Planes between a plane's first and second tiles: more overflow L2, fewer
+    // leave second tiles waiting for planes whose first tiles (2 per resident
+    // CTA) are still in flight.  About 33 MB of planes in complex64 and 26 MB in
+    // complex128, at most 128 planes; 64 for fields of up to 2^20 points.  Per
+    // step with 64 and this many: complex64 128^3 72 and 64 us, 160^3 (real time)
+    // 122 and 112, 192^3 159 and 150; complex128 128^3 97 and 88; 256^3 complex128
+    // with 24 426, 32 433, 64 484.
+    const long plane_bytes = (long)n * n * per * 8;
+    if (c->N > (1L << 20))
+        xc.ctr.lag = (int)std::min<long>(128, ((per == 1 ? 33L : 26L) << 20) / plane_bytes);
     if (const char* lag = std::getenv("GPUE_XY_LAG")) xc.ctr.lag = std::max(1, std::atoi(lag));
     if (const char* w = std::getenv("GPUE_TEST_PLANE_WAIT")) xc.ctr.wait_extra = std::max(0, std::atoi(w));
-    const long tiles = 2L * (n / 16) * c->ax[2].n;
+    const long tiles = 2L * (n / lt) * c->ax[2].n;
     xc.blocks = (int)std::min<long>((long)per_sm * c->sms, tiles);
     xc.k = k;
     return GPUE_OK;
@@ -511,10 +538,14 @@ static bool step_ready(gpue_ctx* c, int prec, int gstate) {
 }
 
 bool plane_ok(const gpue_ctx* c, int prec) {
-    if (c->xy[prec].k && !c->ext)
-        return !(c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1)));
-    if (!c->plane[prec].k || c->ext) return false;
-    return !(c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1)));
+    if (c->ext) return false;
+    const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
+    if (c->xy[prec].k) {
+        if (!gauge) return true;
+        return c->xy[prec].gauge && axis_gauge_active(c, 0) && axis_gauge_active(c, 1) &&
+               (prec == GPUE_PREC_FP64 || c->N >= kTileGaugeMin32);
+    }
+    return c->plane[prec].k && !gauge;
 }
 
 gpue_status make_pass_args(gpue_ctx* c, int prec, const LPass& lp, int gstate, PassArgs& a) {
@@ -552,10 +583,13 @@ gpue_status make_pass_args(gpue_ctx* c, int prec, const LPass& lp, int gstate, P
     a.gscale = 1.0 / (double)c->ax[ax_i].n;
     double axc, ayc;
     gauge_coefs(c, axc, ayc);
-    a.gauge_coef = lp.axis == 0 ? axc : lp.axis == 1 ? ayc : 0.0;
-    a.gauge_src = lp.axis == 0 ? 1 : 0;
+    // the axis whose gauge factor the pass applies
+    const int g_i = lp.axis == kPlaneInvGy ? 1 : lp.axis == kPlaneInvGx ? 0 : lp.axis;
+    a.gauge_coef = g_i == 0 ? axc : g_i == 1 ? ayc : 0.0;
+    a.gauge_src = g_i == 0 ? 1 : 0;
     a.gauge_dt = lp.gauge_dt;
-    a.dmom = c->ax[ax_i].n > 1 ? c->ax[ax_i].p[1] : 0.0;
+    const int m_i = g_i < 3 ? g_i : ax_i;
+    a.dmom = c->ax[m_i].n > 1 ? c->ax[m_i].p[1] : 0.0;
     a.kin_coef = p.hbar * p.hbar / (2 * p.mass);
     for (int i = 0; i < 3; ++i) {
         a.vfac[i] = tb.vfac[i];
@@ -600,7 +634,10 @@ gpue_status make_pass_args(gpue_ctx* c, int prec, const LPass& lp, int gstate, P
 bool tile_pass(gpue_ctx* c, int prec, const LPass& lp, const PassArgs& a, TileLaunch& t) {
     if (lp.axis >= kPlaneFwd && c->xy[prec].k) {
         const XYCfg& xc = c->xy[prec];
-        t.fn = lp.axis == kPlaneFwd ? xc.k->fwd : xc.k->inv;
+        t.fn = lp.axis == kPlaneFwd     ? xc.k->fwd
+               : lp.axis == kPlaneInv   ? xc.k->inv
+               : lp.axis == kPlaneInvGy ? xc.k->inv_gy
+                                        : xc.k->inv_gx;
         t.tm0 = &xc.tmx;
         t.tm1 = &xc.tmy;
         t.kc = xc.ctr.dev();
@@ -708,15 +745,21 @@ void step_passes(gpue_ctx* c, int i, int gstate, bool scale_first, double rexp, 
             if (ord[k] < c->dim && axis_gauge_active(c, ord[k])) gaxes.push_back(ord[k]);
     }
     std::vector<LPass> s;
-    if (plane && c->dim == 3 && gaxes.empty()) {
-        // XY[scale V/2 Fx Fy] Z[Fz K Iz] XY[Ix Iy V/2]
+    if (plane && c->dim == 3 && (gaxes.empty() || (gaxes.size() == 2 && gaxes[0] < 2 && gaxes[1] < 2))) {
+        // XY[scale V/2 Fx Fy] Z[Fz K Iz] XY[Ix Iy V/2], or with the gauge
+        // ..  YX[Iy Ix V/2 F Gx I] Y[F Gy I]  and  XY[Ix Iy V/2 F Gy I] X[F Gx I]
         LPass f = P(kPlaneFwd, {});
         if (scale_first) f.ops.push_back(OP_SCALE);
         s.push_back(f);
         LPass kp = P(2, {OP_FFT_F, OP_KPHASE, OP_FFT_I});
         if (g_apply) kp.kscale_slot = kGuard;
         s.push_back(kp);
-        s.push_back(P(kPlaneInv, {}));
+        if (gaxes.empty()) {
+            s.push_back(P(kPlaneInv, {}));
+        } else {
+            s.push_back(P(gaxes[0] == 0 ? kPlaneInvGx : kPlaneInvGy, {}));
+            s.push_back(P(gaxes[1], {OP_FFT_F, OP_GAUGE, OP_FFT_I}));
+        }
     } else {
         std::vector<int> first;
         if (scale_first) first.push_back(OP_SCALE);
@@ -1496,7 +1539,9 @@ gpue_status ensure_shadow(gpue_ctx* c) {
         gpue_status st = plan_axis(c, GPUE_PREC_FP64, a);
         if (st) return st;
     }
-    return plan_step(c, GPUE_PREC_FP64);
+    gpue_status st = plan_zpass(c, GPUE_PREC_FP64);
+    if (!st) st = plan_xy(c, GPUE_PREC_FP64);
+    return st ? st : plan_step(c, GPUE_PREC_FP64);
 }
 
 // After a polish the FP64 shadow holds the state; bring it back.

@@ -68,8 +68,9 @@ struct PlaneCfg {
     const PlaneKernel* k = nullptr;
     int blocks = 0;
 };
-// LPass::axis values of the two plane passes
-enum { kPlaneFwd = 3, kPlaneInv = 4 };
+// LPass::axis values of the plane passes: forward, inverse, and the inverse
+// with the first gauge pass (along y after x-tiles, along x after y-tiles)
+enum { kPlaneFwd = 3, kPlaneInv = 4, kPlaneInvGy = 5, kPlaneInvGx = 6 };
 
 // Work counters of a tile-stream pass (tstream.cuh): ticket (8 bytes),
 // finish count (4 bytes, padded to 8), one int per z-plane; cleared once at
@@ -77,7 +78,7 @@ enum { kPlaneFwd = 3, kPlaneInv = 4 };
 struct TSCounters {
     void* mem = nullptr;
     size_t bytes = 0;
-    int lag = 64;  // XY pass: planes between a plane's x-tiles and its y-tiles
+    int lag = 64;  // XY pass: planes between a plane's first and second tiles
     // XY pass: x-tiles beyond a plane's own that its y-tiles wait for: 0, or
     // (GPUE_TEST_PLANE_WAIT, for tests only) more than ever come, so every
     // such wait runs out and the run reports GPUE_ERR_TIMEOUT
@@ -99,6 +100,7 @@ struct XYCfg {
     const XYKernel* k = nullptr;
     CUtensorMap tmx, tmy;
     int blocks = 0;
+    bool gauge = false;  // planned for the inverse passes with the gauge
     TSCounters ctr;
 };
 
@@ -297,8 +299,8 @@ void step_passes(gpue_ctx* c, int i, int gstate, bool scale_first, double rexp, 
 // Plans the XY-plane passes of precision prec when the context qualifies
 // (3D, nx = ny with a compiled plane kernel); leaves them off otherwise.
 gpue_status plan_plane(gpue_ctx* c, int prec);
-// Plans the TMA z pass of precision prec when the context qualifies (3D, nx a
-// multiple of 16, nz <= 256 with a compiled kernel).
+// Plans the TMA z pass of precision prec when the context qualifies (3D, a
+// compiled kernel for nz).
 gpue_status plan_zpass(gpue_ctx* c, int prec);
 // Plans the cluster-free XY pass (3D, nx = ny <= 256 with a compiled kernel);
 // when planned it runs the plane passes of the step instead of the cluster

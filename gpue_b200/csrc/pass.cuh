@@ -117,8 +117,8 @@ struct PassArgs {
 struct XYCounters {
     unsigned long long* ticket;  // next ticket
     unsigned* finish;            // CTAs finished
-    int* done_x;                 // [nz] x-tiles stored per plane (XY pass)
-    int lag;                     // XY pass: planes between a plane's x-tiles and y-tiles
+    int* done_x;                 // [nz] first-kind tiles stored per plane (XY pass)
+    int lag;                     // XY pass: planes between a plane's first and second tiles
     int wait_extra;              // XY pass: 0; > 0 only to test the bounded plane wait
 };
 
@@ -297,17 +297,19 @@ __device__ __forceinline__ double decay(double a) {
 
 // OP_VHALF with separable factors: psi *= fa[k] * lf * (nonlinear factor),
 // fa the pass axis' FP64 V/2 factors, lf the product of the other axes' at the
-// line.  The nonlinear angle gN|psi|^2 Dt/(2 hbar) is almost always below 1/16,
+// line; nl_coef as in op_vhalf_f32.  The nonlinear angle gN|psi|^2 Dt/(2 hbar)
+// is almost always below 1/16,
 // where a Taylor series is exact to FP64: that is decided once for the
 // thread's values (an FP32 estimate with margin), so the unrolled loops have
 // no branch and the values' FP64 chains interleave.
 template <typename T, class L>
 __device__ __forceinline__ void op_vhalf_sep(cx<T> (&v)[L::E], int t, const double2* fa,
-                                             cx<double> lf, const PassArgs& a, int gstate) {
+                                             cx<double> lf, const PassArgs& a, int gstate,
+                                             double nl_coef) {
     constexpr int E = L::E;
     bool small = true;
     if (a.gpe) {
-        const float nl = (float)a.nl_coef;
+        const float nl = (float)nl_coef;
         float m = 0.f;
 #pragma unroll
         for (int e = 0; e < E; ++e)
@@ -321,20 +323,20 @@ __device__ __forceinline__ void op_vhalf_sep(cx<T> (&v)[L::E], int t, const doub
     } else if (small && gstate == 0) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const double gd = a.nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
+            const double gd = nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
             v[e] = apply_re(v[e], fa[L::index(t, e)].x * lf.x * taylor_decay(gd));
         }
     } else if (small) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const double gd = a.nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
+            const double gd = nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
             const cx<double> f = cmul(ld2(fa, L::index(t, e)), lf);
             v[e] = apply(v[e], cmul(f, taylor_phase(gd)));
         }
     } else {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const double gd = a.nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
+            const double gd = nl_coef * ((double)v[e].x * v[e].x + (double)v[e].y * v[e].y);
             if (gstate == 0)
                 v[e] = apply_re(v[e], fa[L::index(t, e)].x * lf.x * small_decay<T>(gd));
             else
@@ -758,7 +760,7 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     if constexpr (std::is_same<T, float>::value)
                         op_vhalf_f32<L>(v, t, a.vd[a.axis], line_delta(lf), a, a.gstate, a.nl_coef);
                     else
-                        op_vhalf_sep<T, L>(v, t, a.vfac[a.axis], lf, a, a.gstate);
+                        op_vhalf_sep<T, L>(v, t, a.vfac[a.axis], lf, a, a.gstate, a.nl_coef);
                     break;
                 }
                 case OP_KPHASE: {

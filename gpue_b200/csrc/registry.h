@@ -39,7 +39,7 @@ struct PlaneKernel {
 const PlaneKernel* find_plane_kernel(int prec, int n);
 
 // The TMA z pass (tstream.cuh) for 3D fields with nz = n: tiles of 16
-// x-columns, `threads` threads and `smem` bytes per CTA; a kernel taking
+// x-columns (8 in complex128), `threads` threads and `smem` bytes per CTA; a kernel taking
 // (z-tile tensor map, unused tensor map, PassArgs, counters) (passed as void*
 // here to keep cuda.h out).
 struct ZPassKernel {
@@ -60,6 +60,8 @@ struct XYKernel {
     int smem;
     const void* fwd;
     const void* inv;
+    const void* inv_gy;  // x-tiles Ix, y-tiles Iy V/2 F Gy I
+    const void* inv_gx;  // y-tiles Iy, x-tiles Ix V/2 F Gx I
 };
 const XYKernel* find_xy_kernel(int prec, int n);
 

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                     if constexpr (std::is_same<T, float>::value)
                         op_vhalf_f32<L>(v, t, vx, line_delta(lfv), a, gstate, a.nl_coef);
                     else
-                        op_vhalf_sep<T, L>(v, t, vx, lfv, a, gstate);
+                        op_vhalf_sep<T, L>(v, t, vx, lfv, a, gstate, a.nl_coef);
                     break;
                 case OP_KPHASE: {
                     const double ks = (sp.flags & SP_KGUARD) ? a.kscale * sh->guard : a.kscale;

@@ -1,28 +1,29 @@
-// tstream.cuh -- the complex64 pass kernels of the 3D step that move whole
-// tiles with TMA: the XY pass (both in-plane transforms, x then y, in one
+// tstream.cuh -- the pass kernels of the 3D step that move whole tiles with
+// TMA: the XY pass (both in-plane transforms, x then y or y then x, in one
 // launch) and the z pass (F K I along z).
 //
-// A tile is 16 lines of one kind:
-//   x-tile  16 consecutive rows of one z-plane (a contiguous 16 x nx block)
-//   y-tile  16 adjacent x-columns of one z-plane over all y
-//   z-tile  16 adjacent x-columns of one y-row over all z
+// A tile is LT lines of one kind, 16 in complex64 and 8 in complex128:
+//   x-tile  LT consecutive rows of one z-plane (a contiguous LT x nx block)
+//   y-tile  LT adjacent x-columns of one z-plane over all y
+//   z-tile  LT adjacent x-columns of one y-row over all z
 // It comes in by one cp.async.bulk.tensor load (this GPU's field, no
-// multicast) and goes back, in place, by one bulk tensor store.  y- and
-// z-tiles land with the 128-byte swizzle: their rows are 16 complex64 values
-// (128 bytes), and the swizzle spreads a column over all banks, so the P
+// multicast) and goes back, in place, by one bulk tensor store (complex128
+// x-tiles by untiled bulk copies: their rows pass the 256 elements a box may
+// have).  y- and z-tiles land with the 128-byte swizzle: their rows are LT
+// values (128 bytes), and the swizzle spreads a column over all banks, so the P
 // threads of a line read (and write) their column without conflicts.  Every
 // line's P threads sit in one warp, so the transform's exchanges need only
 // __syncwarp: no compute warp waits for another.
 //
-// Roles: one producer warp (one active lane) and 16 * P / 32 compute warps.
+// Roles: one producer warp (one active lane) and LT * P / 32 compute warps.
 // The producer takes tickets from a grid-wide counter, issues the loads into
 // two landing buffers (full[b], mbarrier with a byte count), waits until the
 // compute warps have written the tile back into its buffer (done[b]), issues
 // the store, and once the buffer has been read out takes the next ticket for
 // it.  The compute warps only wait for full[b].
 //
-// XY ordering.  Tickets follow: the x-tiles of plane g, then the y-tiles of
-// plane g - LAG, for g = 0, 1, ...  A y-tile of plane z may load only after
+// XY ordering (for y then x exchange the two).  Tickets follow: the x-tiles of
+// plane g, then the y-tiles of plane g - LAG, for g = 0, 1, ...  A y-tile of plane z may load only after
 // all x-tiles of plane z are stored (a per-plane count, raised with release
 // semantics by each x-tile's producer once its store is complete, and read
 // with acquire semantics); by then the plane is normally still in L2, so the
@@ -45,9 +46,24 @@
 // no memset between them.
 //
 // Ops.  XY forward: x-tiles [scale] V/2 Fx, y-tiles Fy.  XY inverse: x-tiles
-// Ix, y-tiles Iy V/2 [norm].  z pass: Fz K Iz.  The arithmetic is that of the
-// line pass's complex64 ops (pass.cuh), with the per-stage twiddle table and
-// the factor tables in shared memory.
+// Ix, y-tiles Iy V/2 [norm].  With the rotation gauge the first gauge pass
+// joins the inverse: x-tiles Ix, y-tiles Iy V/2 F Gy I, or y then x: y-tiles Iy,
+// x-tiles Ix V/2 F Gx I (the other axis' gauge pass follows as a line pass).
+// z pass: Fz K Iz.  The arithmetic is that of the line pass's ops (pass.cuh),
+// with the per-stage twiddle table and the factor tables in shared memory.
+//
+// What bounds it.  Complex64: instruction issue (0.50 to 0.55 per scheduler
+// cycle).  Complex128: shared memory, so its 256-point plan is the one with a
+// single exchange (16 x 16, 16 values a thread: 433 us per 256^3 step; 8 x 4 x 8
+// with twice the warps 520).  The z pass then moves 4.9 TB/s, the XY passes 3.2.
+// Per step of 256^3 complex128, five line passes and these three: 809 -> 426 us;
+// 128^3 125 -> 87; with the gauge 256^3 1170 -> 780, complex64 704 -> 506.
+//
+// The norm in complex128: every warp leaves its FP64 sum of a tile with the
+// producer, which adds the warps' in order into the tile's partial; the last CTA
+// to finish sums all tiles' partials in tile order, so the result does not
+// depend on which CTA took which tile and runs repeat bit for bit.  Complex64
+// keeps one compensated sum per thread (the per-tile sums cost 1.2 % there).
 #pragma once
 
 #include <cuda.h>
@@ -59,14 +75,14 @@
 
 namespace gpue {
 
-enum : int { TS_XY_FWD = 0, TS_XY_INV = 1, TS_Z = 2 };
+enum : int { TS_XY_FWD = 0, TS_XY_INV = 1, TS_Z = 2, TS_XY_INV_GY = 3, TS_YX_INV_GX = 4 };
 enum : int { TILE_X = 0, TILE_Y = 1, TILE_Z = 2, TILE_END = -1 };
 
 template <typename T, int N, int RA, int RB, int P, int RC>
 struct TSShape {
     using L = LineFFT<T, N, RA, RB, P, RC>;
     static constexpr int E = L::E;
-    static constexpr int LT = 16;           // lines per tile
+    static constexpr int LT = 128 / (int)sizeof(cx<T>);  // lines per tile
     static constexpr int CT = LT * P;       // compute threads
     static constexpr int CW = CT / 32;      // compute warps
     static constexpr int THREADS = CT + 32; // + the producer warp
@@ -74,16 +90,24 @@ struct TSShape {
     static constexpr int LS = L::LS;
     static constexpr size_t XCH = (size_t)LT * LS * sizeof(cx<T>);
     static constexpr size_t TWB = (size_t)N * 16;
-    static constexpr size_t DB = (size_t)N * sizeof(float2);
+    static constexpr size_t DB = (size_t)N * 2 * sizeof(T);
     static constexpr size_t OFF_XCH = 2 * TILE;
     static constexpr size_t OFF_TW = OFF_XCH + XCH;
     static constexpr size_t OFF_D = OFF_TW + TWB;
     static constexpr size_t OFF_BAR = OFF_D + 2 * DB;
-    // + 4 mbarriers, 2 tile slots and a 256-plane ready bitmap, + 1024 bytes
-    // to align the base (the 128-byte swizzle repeats every 1024 bytes of the
-    // destination address)
-    static constexpr size_t SMEM = OFF_BAR + 96 + 1024;
-    static_assert(std::is_same<T, float>::value, "complex64 tile stream");
+    // + 4 mbarriers, 2 tile slots and a 256-plane ready bitmap, the warps' norm
+    // partials of the two tiles, + 1024 bytes to align the base (the 128-byte
+    // swizzle repeats every 1024 bytes of the destination address)
+    static constexpr size_t OFF_NRM = OFF_BAR + 96;
+    static constexpr size_t SMEM = OFF_NRM + 2 * CW * 8 + 1024;
+    // resident CTAs: complex64 measured no faster with more than two (160^3 in
+    // real time 113 us per step with two, 118 with three); complex128 tiles of
+    // the short lengths hold few warps, so as many as fit
+    static constexpr int BY_SMEM = (int)((size_t)(227 * 1024) / (SMEM + 1024));
+    static constexpr int BY_REGS =
+        65536 / (THREADS * (E <= 4 ? 80 : E <= 8 ? 112 : E <= 12 ? 136 : 200));
+    static constexpr int FIT = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
+    static constexpr int MINB = sizeof(T) == 4 || FIT < 2 ? 2 : FIT;
     static_assert(N <= 256 && N % LT == 0, "a TMA box dimension holds at most 256 elements");
     static_assert(CT % 32 == 0 && 32 % P == 0, "whole warps; a line's threads in one warp");
     static_assert(TILE % 1024 == 0, "landing tiles keep the swizzle alignment");
@@ -91,39 +115,42 @@ struct TSShape {
     static_assert(L::kStageTableLen <= N, "the per-stage twiddle table fits its region");
 };
 
-// Element (row r, column c) of a [rows][16] complex64 tile landed with the
-// 128-byte swizzle: the 16-byte chunk index (c / 2) is XORed with r mod 8.
+// Element (row r, column c) of a [rows][128 bytes] tile landed with the 128-byte
+// swizzle: the 16-byte chunk index is XORed with r mod 8.
+template <typename T>
 __device__ __forceinline__ int sw128(int r, int c) {
-    return r * 16 + ((((c >> 1) ^ (r & 7)) << 1) | (c & 1));
+    if constexpr (sizeof(T) == 4) return r * 16 + ((((c >> 1) ^ (r & 7)) << 1) | (c & 1));
+    else return r * 8 + (c ^ (r & 7));
 }
 
-// XY ticket t -> (kind, plane, tile): xi x-tiles and yi y-tiles per plane
-// (32-bit arithmetic: a launch has nz * (xi + yi) < 2^31 tiles).
-__device__ __forceinline__ int xy_ticket(unsigned t, unsigned xi, unsigned yi, unsigned nz,
-                                         unsigned lag, int& z, int& tile) {
-    const unsigned t1 = lag * xi, t2 = t1 + (nz - lag) * (xi + yi);
+// XY ticket t -> (second kind?, plane, tile): n1 tiles of the first kind and n2
+// of the second per plane (32-bit arithmetic: a launch has nz * (n1 + n2) <
+// 2^31 tiles).
+__device__ __forceinline__ bool xy_ticket(unsigned t, unsigned n1, unsigned n2, unsigned nz,
+                                          unsigned lag, int& z, int& tile) {
+    const unsigned t1 = lag * n1, t2 = t1 + (nz - lag) * (n1 + n2);
     if (t < t1) {
-        z = (int)(t / xi);
-        tile = (int)(t % xi);
-        return TILE_X;
+        z = (int)(t / n1);
+        tile = (int)(t % n1);
+        return false;
     }
     if (t < t2) {
         const unsigned u = t - t1;
-        const int w = (int)(u % (xi + yi));
-        const int g = (int)(lag + u / (xi + yi));
-        if (w < xi) {
+        const int w = (int)(u % (n1 + n2));
+        const int g = (int)(lag + u / (n1 + n2));
+        if (w < (int)n1) {
             z = g;
             tile = w;
-            return TILE_X;
+            return false;
         }
         z = g - lag;
-        tile = w - xi;
-        return TILE_Y;
+        tile = w - n1;
+        return true;
     }
     const unsigned u = t - t2;
-    z = (int)(nz - lag + u / yi);
-    tile = (int)(u % yi);
-    return TILE_Y;
+    z = (int)(nz - lag + u / n2);
+    tile = (int)(u % n2);
+    return true;
 }
 
 // The x-tile count of a plane, read with acquire semantics (the stores it
@@ -162,7 +189,8 @@ __device__ __forceinline__ bool mbar_test(uint64_t* b, unsigned parity) {
 }
 
 template <typename T, int N, int RA, int RB, int P, int RC, int KIND>
-__global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
+__global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS,
+                                  TSShape<T, N, RA, RB, P, RC>::MINB)
     k_tstream(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
               const PassArgs a, const XYCounters k) {
     using S_ = TSShape<T, N, RA, RB, P, RC>;
@@ -173,26 +201,38 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
     unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
     cx<T>* land = reinterpret_cast<cx<T>*>(smem);  // [2] tiles
     cx<T>* xch = reinterpret_cast<cx<T>*>(smem + S_::OFF_XCH);
-    float4* tws = reinterpret_cast<float4*>(smem + S_::OFF_TW);
-    // factor tables: V/2 along x and y (XY), or the K factor along z as
-    // (d.x, d.y, d.y, d.x) for the packed product (z pass)
-    float2* d0_s = reinterpret_cast<float2*>(smem + S_::OFF_D);
-    float2* d1_s = d0_s + N;
+    constexpr bool F32 = std::is_same<T, float>::value;
+    using W = std::conditional_t<F32, float4, double2>;   // a twiddle table entry
+    using Fac = std::conditional_t<F32, float2, double2>; // a factor table entry
+    W* tws = reinterpret_cast<W*>(smem + S_::OFF_TW);
+    // factor tables: V/2 along x and y (XY), or the K factor along z, complex64
+    // as (d.x, d.y, d.y, d.x) for the packed product (z pass)
+    Fac* d0_s = reinterpret_cast<Fac*>(smem + S_::OFF_D);
+    Fac* d1_s = d0_s + N;
     float4* dz_s = reinterpret_cast<float4*>(smem + S_::OFF_D);
+    // the first and second tile kind of an XY pass
+    constexpr bool YX = KIND == TS_YX_INV_GX;
+    constexpr int K1 = YX ? TILE_Y : TILE_X, K2 = YX ? TILE_X : TILE_Y;
+    double* nrm = reinterpret_cast<double*>(smem + S_::OFF_NRM);  // [2][CW]
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S_::OFF_BAR);
     uint64_t* done = full + 2;
     int4* slot = reinterpret_cast<int4*>(smem + S_::OFF_BAR + 32);  // [2] (kind, z, tile)
     unsigned* s_ready = reinterpret_cast<unsigned*>(smem + S_::OFF_BAR + 64);  // planes ready
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    L::build_stage_table(tws, reinterpret_cast<const float4*>(a.tw), tid, S_::THREADS);
+    L::build_stage_table(tws, reinterpret_cast<const W*>(a.tw), tid, S_::THREADS);
     for (int i = tid; i < N; i += S_::THREADS) {
-        if constexpr (KIND == TS_Z) {
+        if constexpr (KIND == TS_Z && F32) {
             const float2 d = a.kd[2][i];
             dz_s[i] = make_float4(d.x, d.y, d.y, d.x);
-        } else {
+        } else if constexpr (KIND == TS_Z) {
+            d0_s[i] = a.kfac[2][i];
+        } else if constexpr (F32) {
             d0_s[i] = a.vd[0][i];
             d1_s[i] = a.vd[1][i];
+        } else {
+            d0_s[i] = a.vfac[0][i];
+            d1_s[i] = a.vfac[1][i];
         }
     }
     if (tid == 0) {
@@ -213,14 +253,16 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
 
     const int nz = a.nz;
     const int xi = a.ny / LT, yi = a.nx / LT;  // x-tiles (and y- or z-tiles) per plane
+    const int n1 = YX ? yi : xi, n2 = YX ? xi : yi;
+    const bool want_norm = KIND != TS_XY_FWD && KIND != TS_Z && a.red.kind == RED_NORM;
     bool ok = true;
-    KSum acc{0.0, 0.0};
+    KSum acc{0.0, 0.0};  // complex64: the thread's norm over its tiles
 
     if (warp == S_::CW) {
         // ------------------------------------------------------ producer
         if (lane == 0) {
             const int lag = k.lag < 1 ? 1 : k.lag < nz ? k.lag : nz;
-            const int need = xi + k.wait_extra;  // x-tiles a plane's y-tiles wait for
+            const int need = n1 + k.wait_extra;  // first tiles a plane's second tiles wait for
             const long total = KIND == TS_Z ? (long)yi * a.ny : (long)nz * (xi + yi);
             // per landing buffer: its ticket and tile, whether its load waits
             // for a plane, the parity of its next done phase, the phases begun
@@ -251,16 +293,27 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
                 return reinterpret_cast<uint64_t>(kd == TILE_Y ? &tm1 : &tm0);
             };
             auto coords = [&](const Buf& m, int& c0, int& c1, int& c2) {
+                // (x in elements of 8 bytes: two per complex128 value)
+                constexpr int per = F32 ? 1 : 2;
                 if (m.kind == TILE_X) {
                     c0 = 0, c1 = m.tile * LT, c2 = m.z;
                 } else if (m.kind == TILE_Y) {
-                    c0 = m.tile * LT, c1 = 0, c2 = m.z;
+                    c0 = m.tile * LT * per, c1 = 0, c2 = m.z;
                 } else {
-                    c0 = m.tile * LT, c1 = m.z, c2 = 0;  // z-tile: z holds the y-row
+                    c0 = m.tile * LT * per, c1 = m.z, c2 = 0;  // z-tile: z holds the y-row
                 }
+            };
+            // complex128 x-tiles: the rows as one contiguous block
+            auto rows_at = [&](const Buf& m) {
+                return static_cast<cx<T>*>(a.out) + ((size_t)m.z * a.ny + (size_t)m.tile * LT) * N;
             };
             auto load = [&](auto bc, Buf& m) {
                 constexpr int b = decltype(bc)::value;
+                if (!F32 && m.kind == TILE_X) {
+                    bulk_load(land + (size_t)b * N * LT, rows_at(m), (unsigned)S_::TILE, full + b);
+                    m.nfull++;
+                    return;
+                }
                 int c0, c1, c2;
                 coords(m, c0, c1, c2);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
@@ -287,10 +340,10 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
                     m.z = (int)((unsigned)m.tk / (unsigned)yi);
                     m.tile = (int)((unsigned)m.tk % (unsigned)yi);
                 } else {
-                    m.kind = xy_ticket((unsigned)m.tk, xi, yi, nz, lag, m.z, m.tile);
+                    m.kind = xy_ticket((unsigned)m.tk, n1, n2, nz, lag, m.z, m.tile) ? K2 : K1;
                 }
                 slot[b] = make_int4(m.kind, m.z, m.tile, 0);
-                if (m.kind == TILE_Y && !known_ready(m.z)) {
+                if (KIND != TS_Z && m.kind == K2 && !known_ready(m.z)) {
                     if (ld_acquire(k.done_x + m.z) < need) {
                         m.pend = true;
                         return;
@@ -324,15 +377,27 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
                     return false;
                 }
                 m.dpar ^= 1u;
-                int c0, c1, c2;
-                coords(m, c0, c1, c2);
-                asm volatile(
-                    "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group "
-                    "[%0, {%1, %2, %3}], [%4];" ::"l"(map_of(m.kind)),
-                    "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(land + (size_t)b * N * LT))
-                    : "memory");
+                if (!F32 && m.kind == TILE_X) {
+                    asm volatile(
+                        "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(rows_at(m)),
+                        "r"(smem_addr(land + (size_t)b * N * LT)), "r"((unsigned)S_::TILE)
+                        : "memory");
+                } else {
+                    int c0, c1, c2;
+                    coords(m, c0, c1, c2);
+                    asm volatile(
+                        "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group "
+                        "[%0, {%1, %2, %3}], [%4];" ::"l"(map_of(m.kind)),
+                        "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(land + (size_t)b * N * LT))
+                        : "memory");
+                }
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                const int stored_x = m.kind == TILE_X ? m.z : -1;
+                if (!F32 && want_norm && m.kind == K2) {
+                    double q = nrm[b * S_::CW];
+                    for (int w = 1; w < S_::CW; ++w) q += nrm[b * S_::CW + w];
+                    a.red.partials[(size_t)m.z * n2 + m.tile] = make_double2(q, 0.0);
+                }
+                const int stored_x = KIND != TS_Z && m.kind == K1 ? m.z : -1;
                 // refill the buffer first: the compute warps wait for it
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 m.tk = (long)nxt;
@@ -396,45 +461,79 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
             const int z = inf.y, tile = inf.z;
             cx<T>* tb = land + (size_t)b * N * LT;
             const bool rows = inf.x == TILE_X;
+            const bool second = KIND != TS_Z && inf.x == K2;
             cx<T> v[E];
             if (rows) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) v[e] = tb[l * N + L::index(t, e)];
             } else {
 #pragma unroll
-                for (int e = 0; e < E; ++e) v[e] = tb[sw128(L::index(t, e), l)];
+                for (int e = 0; e < E; ++e) v[e] = tb[sw128<T>(L::index(t, e), l)];
             }
+            const int line = tile * LT + l;  // y of an x-tile's row, x of a column
+            // V/2 along the tile's lines: o the other in-plane axis' factors
+            auto vhalf = [&](const Fac* d, const double2* o, double s) {
+                const cx<double> lf = cscale(cmul(ld2(o, line), ld2(a.vfac[2], z)), s);
+                // a pending scale is folded into the factor, so the density of
+                // the unscaled values takes it squared
+                const double nl = a.nl_coef * s * s;
+                if constexpr (F32)
+                    op_vhalf_f32<L>(v, t, d, line_delta(lf), a, a.gstate, nl);
+                else
+                    op_vhalf_sep<T, L>(v, t, d, lf, a, a.gstate, nl);
+            };
             if constexpr (KIND == TS_XY_FWD) {
-                if (rows) {
-                    const int y = tile * LT + l;
-                    const cx<double> lf =
-                        cscale(cmul(ld2(a.vfac[1], y), ld2(a.vfac[2], z)), sc);
-                    // the pending scale is folded into the factor, so the
-                    // density of the unscaled values takes it squared
-                    op_vhalf_f32<L>(v, t, d0_s, line_delta(lf), a, a.gstate, a.nl_coef * sc * sc);
-                }
+                if (rows) vhalf(d0_s, a.vfac[1], sc);
                 L::template forward<true>(v, t, sl, twp, sync);
-            } else if constexpr (KIND == TS_XY_INV) {
+            } else if constexpr (KIND == TS_Z) {
+                // z holds the y-row
+                L::template forward<true>(v, t, sl, twp, sync);
+                const cx<double> lf = cmul(ld2(a.kfac[0], line), ld2(a.kfac[1], z));
+                if constexpr (F32)
+                    op_kphase_f32_packed<L>(v, t, dz_s, line_delta(lf), (float)ks);
+                else
+                    op_kphase_f64<L>(v, t, d0_s, cscale(lf, ks), a.gstate);
                 L::template forward<true, true>(v, t, sl, twp, sync);  // inverse
-                if (!rows) {
-                    const int x = tile * LT + l;
-                    const cx<double> lf = cmul(ld2(a.vfac[0], x), ld2(a.vfac[2], z));
-                    op_vhalf_f32<L>(v, t, d1_s, line_delta(lf), a, a.gstate, a.nl_coef);
-                    if (a.red.kind == RED_NORM) op_norm_f32<E>(v, acc);
-                }
             } else {
-                const int x = tile * LT + l;  // z holds the y-row
-                L::template forward<true>(v, t, sl, twp, sync);
-                const cx<double> lf = cmul(ld2(a.kfac[0], x), ld2(a.kfac[1], z));
-                op_kphase_f32_packed<L>(v, t, dz_s, line_delta(lf), (float)ks);
                 L::template forward<true, true>(v, t, sl, twp, sync);  // inverse
+                if (second) {
+                    if constexpr (YX) vhalf(d0_s, a.vfac[1], 1.0);
+                    else vhalf(d1_s, a.vfac[0], 1.0);
+                    if constexpr (KIND != TS_XY_INV) {
+                        // the gauge pass of the second axis (its angle depends
+                        // on the line's coordinate)
+                        L::template forward<true>(v, t, sl, twp, sync);
+                        const double ang =
+                            a.gauge_coef * a.pos[YX ? 1 : 0][line] * a.gauge_dt * a.dmom;
+                        bool small = false;
+                        if constexpr (F32) {
+                            small = gauge_small(ang, N);
+                            if (small) op_gauge_f32<L>(v, t, ang, a.gstate, a.gscale);
+                        }
+                        if (!small)
+                            op_gauge<T, L>(v, gauge_consts<L>(t, ang, a.gstate, a.gscale),
+                                           a.gstate);
+                        __syncwarp();
+                        L::template forward<true, true>(v, t, sl, twp, sync);
+                    }
+                    if (F32 && want_norm) {
+                        if constexpr (F32) op_norm_f32<E>(v, acc);
+                    } else if (want_norm) {
+                        KSum one{0.0, 0.0};
+                        if constexpr (!F32) op_norm<T, E>(v, one);
+                        double q = one.s + one.c;
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
+                        if (lane == 0) nrm[b * S_::CW + warp] = q;
+                    }
+                }
             }
             if (rows) {
 #pragma unroll
                 for (int e = 0; e < E; ++e) tb[l * N + L::index(t, e)] = v[e];
             } else {
 #pragma unroll
-                for (int e = 0; e < E; ++e) tb[sw128(L::index(t, e), l)] = v[e];
+                for (int e = 0; e < E; ++e) tb[sw128<T>(L::index(t, e), l)] = v[e];
             }
             // this thread's writes before the bulk store reads the buffer
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -445,9 +544,32 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS, 2)
     }
     if (!ok && a.err) atomicExch(a.err, 1);
     pdl_launch_dependents();
-    if (KIND == TS_XY_INV && a.red.kind != RED_NONE) {
+    if (F32 && want_norm) {
         __syncthreads();
         grid_reduce_finish(acc, reinterpret_cast<double*>(xch), a.red, gridDim.x, blockIdx.x);
+    } else if (want_norm) {
+        // the last CTA to finish sums the tiles' partials in tile order
+        __shared__ unsigned s_last;
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            s_last = atomicAdd(a.red.counter, 1u) == gridDim.x - 1 ? 1u : 0u;
+        }
+        __syncthreads();
+        if (s_last) {
+            __threadfence();
+            KSum r{0.0, 0.0};
+            const int parts = nz * n2;
+            for (int i = tid; i < parts; i += S_::THREADS) {
+                const double2 q = __ldcg(a.red.partials + i);
+                r.merge(q.x, q.y);
+            }
+            r = block_reduce(r, reinterpret_cast<double*>(xch));
+            if (tid == 0) {
+                a.red.out[0] = sqrt(*a.red.target / (r.s + r.c));
+                *a.red.counter = 0u;
+            }
+        }
     }
 }
 
