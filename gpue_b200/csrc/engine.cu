@@ -505,10 +505,6 @@ gpue_status plan_step(gpue_ctx* c, int prec) {
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     const size_t smem = k->smem(k->lines);
     if (!coop || smem > (size_t)max_smem) return GPUE_OK;
-    if (!c->step_slots) {  // one 16-byte slot per CTA, at most one CTA per row
-        CK(cudaMalloc(&c->step_slots, n * sizeof(double2)));
-        CK(cudaMemsetAsync(c->step_slots, 0, n * sizeof(double2), c->stream));
-    }
     sc.k = k;
     sc.threads = k->lines * k->p;
     sc.blocks = (n + k->lines - 1) / k->lines;
@@ -1509,8 +1505,8 @@ size_t ctx_bytes_estimate(int dim, int n, int prec) {
     const size_t N = (size_t)n * n * (dim == 3 ? n : 1);
     const size_t cap = N / n + kAuxPartials + 1024;  // partials_cap (gpue_ctx_create)
     size_t b = al(N * elem_size(prec)) + al(N * 16);  // state, scratch
-    b += al(kNScal * sizeof(double)) + al(cap * sizeof(double2)) +
-         al(kNCtr * sizeof(unsigned)) + al(4 * sizeof(int));
+    b += al(kNScal * sizeof(double) + 4 * sizeof(int)) + al(cap * sizeof(double2)) +
+         al(256 + (dim == 2 ? (size_t)n * sizeof(double2) : 0));
     const size_t tn = 3 * (2 * al((size_t)n * 16) + al((size_t)n * 16) +
                            3 * al((size_t)n * 8));
     return b + tn;  // one precision's operator tables
@@ -1647,13 +1643,19 @@ gpue_status gpue_ctx_create(const gpue_params* p, gpue_ctx** out) {
     CK(cudaEventCreate(&c->ev1));
     CK(cudaMalloc(&c->psi, c->N * elem_size(c->prec)));
     CK(cudaMalloc(&c->scratch, c->N * 16));
-    CK(cudaMalloc(&c->scal, kNScal * sizeof(double)));
+    // the scalars and, behind them, the flags: one copy reads both back
+    CK(cudaMalloc(&c->scal, kNScal * sizeof(double) + 4 * sizeof(int)));
+    c->dflags = reinterpret_cast<int*>(c->scal + kNScal);
     c->partials_cap = c->N / nx + kAuxPartials + 1024;
     CK(cudaMalloc(&c->partials, c->partials_cap * sizeof(double2)));
-    CK(cudaMalloc(&c->counters, kNCtr * sizeof(unsigned)));
-    CK(cudaMalloc(&c->dflags, 4 * sizeof(int)));
+    // the counters, then the 2D stepper's norm slots (16 bytes per CTA, at most
+    // one CTA per row)
+    static_assert(kNCtr * sizeof(unsigned) <= 256, "slots start at 256");
+    const size_t ctr_bytes = 256 + (c->dim == 2 ? (size_t)nx * sizeof(double2) : 0);
+    CK(cudaMalloc(&c->counters, ctr_bytes));
+    c->step_slots = reinterpret_cast<double2*>(reinterpret_cast<char*>(c->counters) + 256);
     CK(cudaMemsetAsync(c->dflags, 0, 4 * sizeof(int), c->stream));
-    CK(cudaMemsetAsync(c->counters, 0, kNCtr * sizeof(unsigned), c->stream));
+    CK(cudaMemsetAsync(c->counters, 0, ctr_bytes, c->stream));
     double hs[kNScal] = {1.0, 0.0, 0.0, 0.0, 1.0, 1.0 / c->dV, 1.0, 1.0};
     CK(cudaMemcpyAsync(c->scal, hs, sizeof hs, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemsetAsync(c->psi, 0, c->N * elem_size(c->prec), c->stream));
@@ -1696,14 +1698,12 @@ gpue_status gpue_ctx_destroy(gpue_ctx* c) {
     for (auto t : c->atab)
         if (t) cudaFree(t);
     if (c->progs) cudaFree(c->progs);
-    if (c->step_slots) cudaFree(c->step_slots);
     if (c->vtx_ws) cudaFree(c->vtx_ws);
     if (c->obs_dev) cudaFree(c->obs_dev);
     cudaFree(c->scratch);
     cudaFree(c->scal);
     cudaFree(c->partials);
     cudaFree(c->counters);
-    cudaFree(c->dflags);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -2234,16 +2234,25 @@ gpue_status gpue_evolve(gpue_ctx* c, int32_t nsteps, int32_t gstate,
         return GPUE_OK;
     }
     CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
+    // the final norm and the wait flag come back in one copy: each round trip
+    // to the host costs a small run 10 us
+    const int sp = c->polished ? GPUE_PREC_FP64 : c->prec;
+    if (res) {
+        st = norm_to_slot(c, sp, kNorm);
+        if (st) return st;
+    }
+    struct {
+        double scal[kNScal];
+        int flags[4];
+    } back;
+    static_assert(sizeof back == kNScal * sizeof(double) + 4 * sizeof(int), "as on the device");
+    CK(cudaMemcpyAsync(&back, c->scal, sizeof back, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    if (c->plane[c->prec].k || c->xy[c->prec].k || c->zpass[c->prec].k || c->step[c->prec].k) {
-        int gave_up = 0;
-        CK(cudaMemcpy(&gave_up, c->dflags + 3, sizeof gave_up, cudaMemcpyDeviceToHost));
-        if (gave_up) {
-            CK(cudaMemset(c->dflags + 3, 0, sizeof gave_up));
-            return fail(c, GPUE_ERR_TIMEOUT, "a plane pass gave up waiting for its data");
-        }
+    if (back.flags[3]) {
+        CK(cudaMemset(c->dflags + 3, 0, sizeof(int)));
+        return fail(c, GPUE_ERR_TIMEOUT, "a pass gave up waiting for its data");
     }
     if (res) {
         std::memset(res, 0, sizeof *res);
@@ -2253,10 +2262,7 @@ gpue_status gpue_evolve(gpue_ctx* c, int32_t nsteps, int32_t gstate,
         res->energy = lo.energy;
         res->device_ms = ms;
         res->kernel_launches = c->launches;
-        double nrm = 0;
-        st = norm_now(c, c->polished ? GPUE_PREC_FP64 : c->prec, &nrm);
-        if (st) return st;
-        res->norm = nrm;
+        res->norm = back.scal[kNorm] * c->dV;
     }
     return GPUE_OK;
 }
