@@ -70,46 +70,103 @@ __device__ __forceinline__ double gauge_energy(const EnergyArgs& a, const cx<T>*
     return px * ir + py * ii;
 }
 
-template <typename T>
-__device__ __forceinline__ KSum energy_real_points(const EnergyArgs& a, long g0, long gstep) {
+// Rows of nx points dealt to `ncta` CTAs of 256 threads: tpr threads (a power of
+// two) share a row and a thread takes B rows at a time, whose loads are requested
+// together.  The y and z indices advance by addition.  f(psi value, x, y, z, flat
+// index) for every point, done() after each batch of rows.
+template <int B, typename T, class F, class D>
+__device__ __forceinline__ void for_rows(const cx<T>* psi, int nx, int ny, int rows, int cta,
+                                         int ncta, F f, D done) {
+    int tpr = 32;
+    while (tpr < nx && tpr < 256) tpr *= 2;
+    const int per = 256 / tpr, lane = (int)threadIdx.x & (tpr - 1);
+    const int step = ncta * per;  // rows per round of all CTAs
+    const int dy = step % ny, dz = step / ny;
+    const long stride = (long)step * nx;
+    int row = cta * per + (int)threadIdx.x / tpr;
+    int y = row % ny, z = row / ny;
+    for (; row < rows; row += B * step) {
+        int yk[B], zk[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            yk[k] = y;
+            zk[k] = z;
+            y += dy;
+            z += dz;
+            if (y >= ny) {
+                y -= ny;
+                ++z;
+            }
+        }
+        const int full = (rows - row + step - 1) / step;  // rows of the batch in the field
+        for (int x = lane; x < nx; x += tpr) {
+            const long g = (long)row * nx + x;
+            cx<T> p[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) p[k] = k < full ? psi[g + k * stride] : cx<T>{(T)0, (T)0};
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if (k < full) f(p[k], x, yk[k], zk[k], g + k * stride);
+        }
+        done();
+    }
+}
+
+// PLAIN: separable V and no gauge term, the form of most checks, in few enough
+// registers for four CTAs per SM and four rows in flight per thread: 256^3 takes
+// 55 us in complex64 and 61 in complex128.  With the gauge term's six divisions
+// per point inlined beside it the kernel held one CTA per SM (224 us); one point
+// at a time with 64-bit index divisions it took 112 us.
+template <typename T, bool PLAIN>
+__device__ __forceinline__ KSum energy_real_points(const EnergyArgs& a, int cta, int ncta) {
     const cx<T>* psi = reinterpret_cast<const cx<T>*>(a.psi);
     const double s = a.scale ? *a.scale : 1.0;
+    const double hg = a.gpe ? 0.5 * a.gN : 0.0;
     const long nxy = (long)a.nx * a.ny;
     KSum acc{0.0, 0.0};
-    for (long g = g0; g < a.N; g += gstep) {
-        const int xi = (int)(g % a.nx);
-        const int yi = (int)((g / a.nx) % a.ny);
-        const int zi = (int)(g / nxy);
-        const cx<T> pv = psi[g];
-        const double px = s * (double)pv.x, py = s * (double)pv.y;
-        const double r = px * px + py * py;
-        const double V = a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-        double e = a.gpe ? r * (V + 0.5 * a.gN * r) : r * V;
-        if (a.lterm) e += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
-        acc.add(e);
-    }
+    double part = 0.0;  // a batch's terms in plain FP64, then into the compensated sum
+    for_rows<PLAIN ? 4 : 1>(
+        psi, a.nx, a.ny, (int)(a.N / a.nx), cta, ncta,
+        [&](cx<T> pv, int xi, int yi, int zi, long g) {
+            const double px = s * (double)pv.x, py = s * (double)pv.y;
+            const double r = px * px + py * py;
+            if constexpr (PLAIN) {
+                const double V = a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
+                part += r * (V + hg * r);
+            } else {
+                const double V =
+                    a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
+                part += r * (V + hg * r);
+                if (a.lterm) part += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+            }
+        },
+        [&] {
+            acc.add(part);
+            part = 0.0;
+        });
     return acc;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_energy_real(const EnergyArgs a) {
+template <typename T, bool PLAIN>
+__global__ void __launch_bounds__(256, PLAIN ? 4 : 2) k_energy_real(const EnergyArgs a) {
     __shared__ double scratch[16];
-    KSum acc = energy_real_points<T>(a, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                                     (long)gridDim.x * blockDim.x);
+    KSum acc = energy_real_points<T, PLAIN>(a, blockIdx.x, gridDim.x);
     grid_reduce_finish(acc, scratch, a.red, gridDim.x, blockIdx.x);
 }
 
 // Independent solves at once: `per` CTAs per solve, each solve reducing over
 // its own CTAs; converged solves (*active == 0) are skipped.
 template <typename T>
-__global__ void __launch_bounds__(256) k_energy_real_batch(const EnergyArgs* __restrict__ args,
+__global__ void __launch_bounds__(256, 3) k_energy_real_batch(const EnergyArgs* __restrict__ args,
                                                           const int* const* __restrict__ active,
                                                           int per) {
     __shared__ double scratch[16];
     const int s = blockIdx.x / per, b = blockIdx.x % per;
     if (active[s] && *active[s] == 0) return;
     const EnergyArgs& a = args[s];
-    KSum acc = energy_real_points<T>(a, (long)b * blockDim.x + threadIdx.x, (long)per * blockDim.x);
+    const bool plain = !a.lterm && !a.vtab;
+    KSum acc = plain ? energy_real_points<T, true>(a, b, per)
+                     : energy_real_points<T, false>(a, b, per);
     grid_reduce_finish(acc, scratch, a.red, per, b);
 }
 
@@ -135,7 +192,7 @@ __device__ __forceinline__ double trapz_w(int i, int n) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_observables(const ObsArgs o) {
+__global__ void __launch_bounds__(256, 2) k_observables(const ObsArgs o) {
     __shared__ double scratch[kObsN][16];
     __shared__ unsigned s_last;
     const EnergyArgs& a = o.e;
@@ -145,37 +202,43 @@ __global__ void __launch_bounds__(256) k_observables(const ObsArgs o) {
     KSum acc[kObsN];
 #pragma unroll
     for (int q = 0; q < kObsN; ++q) acc[q] = KSum{0.0, 0.0};
-    for (long g = (long)blockIdx.x * blockDim.x + threadIdx.x; g < a.N;
-         g += (long)gridDim.x * blockDim.x) {
-        const int xi = (int)(g % a.nx);
-        const int yi = (int)((g / a.nx) % a.ny);
-        const int zi = (int)(g / nxy);
-        const cx<T> pv = psi[g];
-        const double px = s * (double)pv.x, py = s * (double)pv.y;
-        const double r = px * px + py * py;
-        const double V = a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-        acc[kObsNorm].add(r);
-        acc[kObsPot].add(r * V);
-        if (a.gpe) acc[kObsInt].add(0.5 * a.gN * r * r);
-        if (a.lterm) acc[kObsRot].add(gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py));
-        const double X = a.pos[0][xi];
-        const double Y = a.dim > 1 ? a.pos[1][yi] : 0.0;
-        const double Z = a.dim > 2 ? a.pos[2][zi] : 0.0;
-        const double wr = r * trapz_w(xi, a.nx) * trapz_w(yi, a.ny) * trapz_w(zi, a.nz);
-        acc[kObsX].add(wr * X);
-        acc[kObsY].add(wr * Y);
-        acc[kObsZ].add(wr * Z);
-        acc[kObsR2].add(wr * (X * X + Y * Y));
-        acc[kObsQ].add(wr * (X * X - Y * Y));
-        if (a.dim > 1) {
-            // -i hbar (x d+y - y d+x) psi, then Re[conj(p) * that]
-            double dxr, dxi, dyr, dyi;
-            dfwd(psi, a.N, g, 1, s, px, py, a.dx, dxr, dxi);
-            dfwd(psi, a.N, g, a.nx, s, px, py, a.dy, dyr, dyi);
-            const double Dr = X * dyr - Y * dxr, Di = X * dyi - Y * dxi;
-            acc[kObsLz].add(a.hbar * (px * Di - py * Dr));
-        }
-    }
+    double part[kObsN] = {};  // a batch's terms in plain FP64
+    for_rows<1>(
+        psi, a.nx, a.ny, (int)(a.N / a.nx), blockIdx.x, gridDim.x,
+        [&](cx<T> pv, int xi, int yi, int zi, long g) {
+            const double px = s * (double)pv.x, py = s * (double)pv.y;
+            const double r = px * px + py * py;
+            const double V =
+                a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
+            part[kObsNorm] += r;
+            part[kObsPot] += r * V;
+            if (a.gpe) part[kObsInt] += 0.5 * a.gN * r * r;
+            if (a.lterm) part[kObsRot] += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+            const double X = a.pos[0][xi];
+            const double Y = a.dim > 1 ? a.pos[1][yi] : 0.0;
+            const double Z = a.dim > 2 ? a.pos[2][zi] : 0.0;
+            const double wr = r * trapz_w(xi, a.nx) * trapz_w(yi, a.ny) * trapz_w(zi, a.nz);
+            part[kObsX] += wr * X;
+            part[kObsY] += wr * Y;
+            part[kObsZ] += wr * Z;
+            part[kObsR2] += wr * (X * X + Y * Y);
+            part[kObsQ] += wr * (X * X - Y * Y);
+            if (a.dim > 1) {
+                // -i hbar (x d+y - y d+x) psi, then Re[conj(p) * that]
+                double dxr, dxi, dyr, dyi;
+                dfwd(psi, a.N, g, 1, s, px, py, a.dx, dxr, dxi);
+                dfwd(psi, a.N, g, a.nx, s, px, py, a.dy, dyr, dyi);
+                const double Dr = X * dyr - Y * dxr, Di = X * dyi - Y * dxi;
+                part[kObsLz] += a.hbar * (px * Di - py * Dr);
+            }
+        },
+        [&] {
+#pragma unroll
+            for (int q = 0; q < kObsN; ++q) {
+                acc[q].add(part[q]);
+                part[q] = 0.0;
+            }
+        });
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int q = 0; q < kObsN; ++q) {
@@ -206,16 +269,25 @@ __global__ void __launch_bounds__(256) k_observables(const ObsArgs o) {
     __syncthreads();
     if (!s_last) return;
     __threadfence();
+    // one warp per quantity: lanes stride over the CTAs' partials (one thread
+    // walking them in turn took a third of the kernel on a 768^2 state)
     __shared__ double fin[kObsN];
-    if (threadIdx.x < kObsN) {
-        const int q = threadIdx.x;
+    for (int q = w; q < kObsN; q += nw) {
         KSum t{0.0, 0.0};
-        for (unsigned i = 0; i < gridDim.x; ++i) {
+        for (unsigned i = lane; i < gridDim.x; i += 32) {
             const double2 p = __ldcg(o.partials + (long)q * gridDim.x + i);
             t.merge(p.x, p.y);
         }
-        fin[q] = t.s + t.c;
-        o.out[q] = fin[q];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const double os = __shfl_down_sync(0xffffffffu, t.s, off);
+            const double oc = __shfl_down_sync(0xffffffffu, t.c, off);
+            t.merge(os, oc);
+        }
+        if (lane == 0) {
+            fin[q] = t.s + t.c;
+            o.out[q] = fin[q];
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -287,16 +359,32 @@ static __global__ void k_batch_gather(const CheckArgs* __restrict__ args, int n,
     }
 }
 
-// sum |psi|^2 (optionally times *scale^2) -> RED_SUM/RED_NORM
+// sum |psi|^2 -> RED_SUM/RED_NORM; with scale, psi *= *scale first (stored), one
+// read of the field instead of two
 template <typename T>
-__global__ void __launch_bounds__(256) k_norm(const void* psi_, long N, RedArgs red) {
+__global__ void __launch_bounds__(256) k_norm(void* psi_, long N, const double* scale,
+                                              RedArgs red) {
     __shared__ double scratch[16];
-    const cx<T>* psi = reinterpret_cast<const cx<T>*>(psi_);
+    cx<T>* psi = reinterpret_cast<cx<T>*>(psi_);
+    const T s = scale ? (T)*scale : (T)1;
+    const long step = (long)gridDim.x * blockDim.x;
     KSum acc{0.0, 0.0};
-    for (long g = (long)blockIdx.x * blockDim.x + threadIdx.x; g < N;
-         g += (long)gridDim.x * blockDim.x) {
-        const cx<T> v = psi[g];
-        acc.add((double)v.x * v.x + (double)v.y * v.y);
+    for (long g = (long)blockIdx.x * blockDim.x + threadIdx.x; g < N; g += 4 * step) {
+        cx<T> v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            v[k] = g + k * step < N ? psi[g + k * step] : cx<T>{(T)0, (T)0};
+        if (scale) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                v[k] = cscale(v[k], s);
+                if (g + k * step < N) psi[g + k * step] = v[k];
+            }
+        }
+        double part = 0.0;  // four terms in plain FP64, then into the compensated sum
+#pragma unroll
+        for (int k = 0; k < 4; ++k) part += (double)v[k].x * v[k].x + (double)v[k].y * v[k].y;
+        acc.add(part);
     }
     grid_reduce_finish(acc, scratch, red, gridDim.x, blockIdx.x);
 }

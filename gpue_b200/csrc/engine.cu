@@ -890,6 +890,12 @@ EnergyArgs energy_args(gpue_ctx* c, int prec, bool scale_pending) {
     return e;
 }
 
+// CTAs of the observables reduction: about 1024 points each at least
+static int obs_blocks(const gpue_ctx* c) {
+    const long most = std::min<long>(c->sms * 2, (kAuxPartials - kObsN) / kObsN);
+    return (int)std::max(1L, std::min(most, c->N / 1024));
+}
+
 // after_pass: the energy passes follow a pass kernel in the stream
 gpue_status launch_energy(gpue_ctx* c, int prec, int gstate, bool scale_pending,
                           bool after_pass = false) {
@@ -910,13 +916,19 @@ gpue_status launch_energy(gpue_ctx* c, int prec, int gstate, bool scale_pending,
         oa.counter = e.red.counter;
         oa.out = c->obs_dev;
         oa.ereal = c->scal + kEreal;
-        const int blocks = (int)std::min<long>(c->sms * 2, (kAuxPartials - kObsN) / kObsN);
+        const int blocks = obs_blocks(c);
         if (prec == GPUE_PREC_FP32) k_observables<float><<<blocks, 256, 0, c->stream>>>(oa);
         else k_observables<double><<<blocks, 256, 0, c->stream>>>(oa);
     } else {
-        const int blocks = c->sms * 4;
-        if (prec == GPUE_PREC_FP32) k_energy_real<float><<<blocks, 256, 0, c->stream>>>(e);
-        else k_energy_real<double><<<blocks, 256, 0, c->stream>>>(e);
+        const int blocks = (int)std::max(1L, std::min<long>(c->sms * 4, c->N / 1024));
+        const bool f32 = prec == GPUE_PREC_FP32;
+        if (!e.lterm && !e.vtab) {
+            if (f32) k_energy_real<float, true><<<blocks, 256, 0, c->stream>>>(e);
+            else k_energy_real<double, true><<<blocks, 256, 0, c->stream>>>(e);
+        } else {
+            if (f32) k_energy_real<float, false><<<blocks, 256, 0, c->stream>>>(e);
+            else k_energy_real<double, false><<<blocks, 256, 0, c->stream>>>(e);
+        }
     }
     c->launches++;
     CK(cudaGetLastError());
@@ -976,8 +988,9 @@ gpue_status apply_pending_scale(gpue_ctx* c, int prec) {
     return GPUE_OK;
 }
 
-// sum |psi|^2 of a state into a scalar slot (stream-ordered, no sync)
-gpue_status norm_to_slot(gpue_ctx* c, int prec, int slot) {
+// sum |psi|^2 of a state into a scalar slot (stream-ordered, no sync); with
+// scale_slot >= 0 the state is scaled by that slot first, in the same pass
+gpue_status norm_to_slot(gpue_ctx* c, int prec, int slot, int scale_slot) {
     RedArgs r;
     std::memset(&r, 0, sizeof r);
     r.kind = RED_SUM;
@@ -985,8 +998,11 @@ gpue_status norm_to_slot(gpue_ctx* c, int prec, int slot) {
     r.counter = c->counters + kCtrMisc;
     r.out = c->scal + slot;
     void* psi = state_of(c, prec);
-    if (prec == GPUE_PREC_FP32) k_norm<float><<<c->sms * 4, 256, 0, c->stream>>>(psi, c->N, r);
-    else k_norm<double><<<c->sms * 4, 256, 0, c->stream>>>(psi, c->N, r);
+    const double* scale = scale_slot >= 0 ? c->scal + scale_slot : nullptr;
+    // (a thread takes four points at a time; fewer partials to sum on small fields)
+    const int blocks = (int)std::max(1L, std::min<long>(c->sms * 4, c->N / 1024));
+    if (prec == GPUE_PREC_FP32) k_norm<float><<<blocks, 256, 0, c->stream>>>(psi, c->N, scale, r);
+    else k_norm<double><<<blocks, 256, 0, c->stream>>>(psi, c->N, scale, r);
     c->launches++;
     CK(cudaGetLastError());
     return GPUE_OK;
@@ -1803,7 +1819,7 @@ gpue_status gpue_observables_get(gpue_ctx* c, gpue_observables* o) {
     std::memset(&oa, 0, sizeof oa);
     oa.e = energy_args(c, sp, c->pending_scale);
     double2* aux = c->partials + (c->partials_cap - kAuxPartials);
-    const int blocks = (int)std::min<long>(c->sms * 2, (kAuxPartials - kObsN) / kObsN);
+    const int blocks = obs_blocks(c);
     oa.partials = aux;
     oa.counter = c->counters + kCtrMisc;
     oa.out = reinterpret_cast<double*>(aux + (long)kObsN * blocks);
@@ -2198,7 +2214,14 @@ gpue_status gpue_evolve(gpue_ctx* c, int32_t nsteps, int32_t gstate,
     LoopOut lo;
     st = step_loop(c, c->prec, off, nsteps, gstate, o, guard, lo);
     if (st) return st;
-    st = apply_pending_scale(c, c->prec);
+    // (the norm of a run that ends here comes with the final renormalisation)
+    const bool scaled_norm = c->pending_scale && res && !o.no_sync && !guard && !polish;
+    if (scaled_norm) {
+        st = norm_to_slot(c, c->prec, kNorm, kScale);
+        c->pending_scale = false;
+    } else {
+        st = apply_pending_scale(c, c->prec);
+    }
     if (st) return st;
     // a guard factor computed by the last step has not been applied yet
     const int last = off + lo.done - 1;
@@ -2237,7 +2260,7 @@ gpue_status gpue_evolve(gpue_ctx* c, int32_t nsteps, int32_t gstate,
     // the final norm and the wait flag come back in one copy: each round trip
     // to the host costs a small run 10 us
     const int sp = c->polished ? GPUE_PREC_FP64 : c->prec;
-    if (res) {
+    if (res && !scaled_norm) {
         st = norm_to_slot(c, sp, kNorm);
         if (st) return st;
     }

@@ -333,7 +333,7 @@ std::vector<LPass> energy_passes(const gpue_ctx* c, bool scale_pending);
 EnergyArgs energy_args(gpue_ctx* c, int prec, bool scale_pending);
 gpue_status scale_state(gpue_ctx* c, int prec, int slot);
 gpue_status apply_pending_scale(gpue_ctx* c, int prec);
-gpue_status norm_to_slot(gpue_ctx* c, int prec, int slot);
+gpue_status norm_to_slot(gpue_ctx* c, int prec, int slot, int scale_slot = -1);
 gpue_status unpolish(gpue_ctx* c);
 // device bytes a context holds (state, scratch, tables, reduction buffers),
 // and the same for a fresh context of the given shape and precision

@@ -10,10 +10,11 @@
 // of plaquette p among the in-radius plaquettes and r_nc(p) the rank of the
 // last non-candidate before it (-1 if none), a candidate is marked iff
 // r(p) - r_nc(p) is odd.  Both ranks are prefix counts, so the finder runs as
-// five small kernels with no serial walk:
-//   k_vtx_winding  one warp per row: candidate code (signed lround of the
-//                  winding, 0 for none) per plaquette, in-radius count and
-//                  rank of the row's last non-candidate;
+// small kernels with no serial walk:
+//   k_vtx_code     one thread per plaquette: candidate code (signed lround of
+//                  the winding, 0 for none);
+//   k_vtx_ranks    one warp per row: in-radius count and rank of the row's
+//                  last non-candidate;
 //   k_vtx_rows     one warp: row offsets of the ranks and, per row, the rank
 //                  of the last non-candidate in the rows before it;
 //   k_vtx_mark     one warp per row: ballots give each candidate's ranks; the
@@ -80,11 +81,21 @@ __device__ __forceinline__ int rank_of_top(unsigned m, unsigned mask_in, int bas
     return base + __popc(mask_in & lanes_below(top));
 }
 
+// One thread per plaquette: four atan2 of dependent FP64 chains each, so every
+// plaquette gets a thread of its own (as one warp walking a row the 768^2 case
+// took 36 us).
 template <typename T>
-__global__ void __launch_bounds__(128) k_vtx_winding(const void* psi_, const double* x, int n,
-                                                     double radius, signed char* code, int* cnt,
-                                                     int* lastnc) {
+__global__ void __launch_bounds__(128) k_vtx_code(const void* psi_, const double* x, int n,
+                                                  double radius, signed char* code) {
     const cx<T>* psi = reinterpret_cast<const cx<T>*>(psi_);
+    const int j = blockIdx.x * 128 + threadIdx.x, i = blockIdx.y;
+    if (j >= n) return;
+    const bool inr = i < n - 1 && j < n - 1 && in_radius(x, i, j, radius);
+    code[(long)i * n + j] = (signed char)(inr ? plaquette_code<T>(psi, n, i, j) : 0);
+}
+
+__global__ void __launch_bounds__(128) k_vtx_ranks(const signed char* code, const double* x,
+                                                   int n, double radius, int* cnt, int* lastnc) {
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5);
     if (i >= n) return;
@@ -92,10 +103,9 @@ __global__ void __launch_bounds__(128) k_vtx_winding(const void* psi_, const dou
     for (int j0 = 0; j0 < n; j0 += 32) {
         const int j = j0 + lane;
         const bool inr = i < n - 1 && j < n - 1 && in_radius(x, i, j, radius);
-        const int cd = inr ? plaquette_code<T>(psi, n, i, j) : 0;
-        if (j < n) code[(long)i * n + j] = (signed char)cd;
         const unsigned mask_in = __ballot_sync(0xffffffffu, inr);
-        const unsigned mask_nc = __ballot_sync(0xffffffffu, inr && cd == 0);
+        const unsigned mask_nc =
+            __ballot_sync(0xffffffffu, inr && code[(long)i * n + j] == 0);
         if (mask_nc) last = rank_of_top(mask_nc, mask_in, rank);
         rank += __popc(mask_in);
     }
@@ -268,10 +278,12 @@ gpue_status gpue_find_vortices(gpue_ctx* c, double radius, int32_t* marker, int3
     const double* x = c->tab[sp].pos[0];
     const void* psi = state_of(c, sp);
     const int blocks = (n + kRowsPerBlock - 1) / kRowsPerBlock;
+    const dim3 points((n + 127) / 128, n);
     if (sp == GPUE_PREC_FP32)
-        k_vtx_winding<float><<<blocks, 128, 0, c->stream>>>(psi, x, n, radius, code, cnt, lastnc);
+        k_vtx_code<float><<<points, 128, 0, c->stream>>>(psi, x, n, radius, code);
     else
-        k_vtx_winding<double><<<blocks, 128, 0, c->stream>>>(psi, x, n, radius, code, cnt, lastnc);
+        k_vtx_code<double><<<points, 128, 0, c->stream>>>(psi, x, n, radius, code);
+    k_vtx_ranks<<<blocks, 128, 0, c->stream>>>(code, x, n, radius, cnt, lastnc);
     k_vtx_rows<<<1, 32, 0, c->stream>>>(cnt, lastnc, n, rowstart, carry);
     k_vtx_mark<<<blocks, 128, 0, c->stream>>>(code, x, n, radius, rowstart, carry, dmarker,
                                               rowfound);
