@@ -14,8 +14,8 @@ One bench step = one gpue_evolve call of 100 imaginary time steps of the fused
 complex64 form through the C ABI (three full-field passes per time step: the
 XY-plane pass, the z pass with the kinetic phase, the inverse XY-plane pass),
 timed with CUDA events on the library's stream.  The same protocol times the
-plain FP64 form (five line passes per step) for the fused-FP32 vs plain-FP64
-ratio.  Extra legs: end to end through the C ABI with host buffers, the full
+plain FP64 form (the same three passes in complex128) for the fused-FP32 vs
+plain-FP64 ratio.  Extra legs: end to end through the C ABI with host buffers, the full
 5000-step relaxation per form with its energies, the 1024^2 rotating
 real-time case, the 256^2 FP64 ground state (10,000 steps), the 96-solve
 batched sweep and the serving stream.
@@ -60,7 +60,7 @@ ROT_NAME = ("2D real-time rotating condensate 1024^2 on [-16,16)^2, g=500, Omega
 SMALL = dict(dim=2, n=256, box=10.0, g=100.0, gdt=1e-4, steps=10000, every=1000, seed=1)
 FLUSH_BYTES = 256 << 20
 # passes per time step of each form on the headline workload
-PASSES = {"fp32": 3, "fp64": 5}
+PASSES = {"fp32": 3, "fp64": 3}
 
 
 def parse_args():
@@ -751,10 +751,9 @@ def profile_case(args):
                           "launches": st1["kernel_launches"], "device_ms": st1["device_ms"]}))
         return
     if args.profile.endswith("_3d"):
-        # the headline workload with fixed launch shapes for the z pass (and
-        # the x/y line passes of the FP64 form), so a capture does not depend
-        # on timings taken under the profiler; one step is one imaginary time
-        # step (3 passes complex64, 5 passes complex128)
+        # the headline workload with fixed launch shapes for the line passes of
+        # the energy checks, so a capture does not depend on timings taken
+        # under the profiler; one step is one imaginary time step (3 passes)
         prec = G.PREC_FP32 if args.profile == "fp32_3d" else G.PREC_FP64
         with G.Solver(head_params(G, prec)) as s:
             for axis, lines in enumerate((2, 4, 4)):

@@ -314,6 +314,10 @@ gpue_status gpue_ctx_wfc_device(gpue_ctx* ctx, void** psi, int32_t* dtype);
  * fastest (by a clear margin over the default) is kept.  Choices are cached per (precision,
  * dimension, length, axis) for the process, so later contexts of the same
  * shape reuse them without timing; flags bit 0 re-times a cached shape.
+ * The line passes are what is tuned: they run 3D steps without tile kernels,
+ * batched solves of such shapes, energy checks, and per-step fields; 2D steps
+ * run on the resident steppers and 3D ones on the tile passes, which have one
+ * shape per length.
  * Setting GPUE_AUTOTUNE=1 in the environment makes gpue_ctx_create do this. */
 gpue_status gpue_autotune(gpue_ctx* ctx, int32_t flags);
 
@@ -342,8 +346,11 @@ gpue_status gpue_list_plans(int32_t precision, int32_t n, gpue_plan_info* out, i
  * stream, so no launch overlaps the next), and then undone: the state and the
  * scalar slots are saved first and put back after.  us[i] receives the mean
  * duration of pass i of a step, kinds[i] what the pass is: 0, 1, 2 a line
- * pass along x, y, z (2 also the z tile pass of a 3D complex64 step), 3 and
- * 4 the forward and inverse XY pass of a 3D complex64 step.  *npass receives
+ * pass along x, y, z (2 also the z tile pass of a 3D step), 3 and 4 the forward
+ * and inverse XY pass of a 3D step, 5 and 6 the inverse XY pass with the
+ * rotation gauge along y and along x.  2D steps run as one resident launch
+ * for many steps; what is timed then are the line passes that do the same
+ * work.  *npass receives
  * the passes per step; at most cap entries are written.  A measurement aid:
  * the results of later calls do not change. */
 gpue_status gpue_time_passes(gpue_ctx* ctx, int32_t gstate, int32_t nsteps, float* us,
@@ -352,7 +359,9 @@ gpue_status gpue_time_passes(gpue_ctx* ctx, int32_t gstate, int32_t nsteps, floa
 /* Use the compiled plan (ra, rb, rc, threads_per_line) on one axis of the
  * context, with lines_per_cta lines per CTA (0: the default count).  Fails
  * with GPUE_ERR_INVALID_ARG when no such plan exists or the launch shape does
- * not fit the grid.  Results differ from another plan's only by round-off. */
+ * not fit the grid.  Results differ from another plan's only by round-off.  A
+ * 2D context whose plan was set runs its steps as line passes with it from
+ * then on, instead of the resident stepper. */
 gpue_status gpue_set_plan(gpue_ctx* ctx, int32_t axis, int32_t ra, int32_t rb, int32_t rc,
                           int32_t threads_per_line, int32_t lines_per_cta);
 
