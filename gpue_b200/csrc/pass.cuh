@@ -655,7 +655,7 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
         t = threadIdx.x % P;
         c = threadIdx.x / P;
     }
-    cx<T>* sl = reinterpret_cast<cx<T>*>(smem_raw) + c * L::LS;
+    cx<T>* sl = reinterpret_cast<cx<T>*>(smem_raw) + c * (STRIDED ? L::LSC : L::LS);
 
     auto sync = [] {
         if constexpr (STRIDED || P > 32) __syncthreads();

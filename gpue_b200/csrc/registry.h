@@ -88,7 +88,7 @@ const PassKernel* pass_table_f64_a(int* count);
 const PassKernel* pass_table_f64_b(int* count);
 
 #define GPUE_PLAN4(T, N, RA, RB, RC, P, MAXT, MINB)                                        \
-    PassKernel{N, RA, RB, RC, P, LineFFT<T, N, RA, RB, P, RC>::LS, (int)sizeof(cx<T>), MAXT,   \
+    PassKernel{N, RA, RB, RC, P, LineFFT<T, N, RA, RB, P, RC>::LSMAX, (int)sizeof(cx<T>), MAXT,\
                &k_pass<T, N, RA, RB, P, false, false, RC, MAXT, MINB>,                       \
                &k_pass<T, N, RA, RB, P, true, false, RC, MAXT, MINB>,                        \
                &k_pass<T, N, RA, RB, P, false, true, RC, MAXT, MINB>,                        \

@@ -86,10 +86,15 @@ struct alignas(16) StepShared {
     double scratch[2 * (512 / 32)];
 };
 
-template <typename T, int N, int RA, int RB, int RC, int P>
+template <typename T, int N, int RA, int RB, int RC, int P, int C>
 struct StepShape {
     using L = LineFFT<T, N, RA, RB, P, RC>;
     static constexpr int E = L::E;
+    // line stride: the C columns a warp touches at once (16 or 8 lanes at a time)
+    // on distinct banks
+    static constexpr int W = sizeof(T) == 4 ? 16 : 8;
+    static constexpr int C2 = C <= 1 ? 1 : C <= 2 ? 2 : C <= 4 ? 4 : C <= 8 ? 8 : 16;
+    static constexpr int LS = L::kPad16 + (W / C2 > 1 ? W / C2 : 1);
     // the per-stage twiddle table and the V/2 (x) and K (y) factors: 1024
     // complex128 points leave no room for the factors beside the exchange
     static constexpr bool FAC = sizeof(T) == 4 || N <= 768;
@@ -99,8 +104,8 @@ struct StepShape {
     static constexpr size_t FACB = FAC ? (size_t)N * 2 * sizeof(T) : 0;  // one factor table
     static constexpr size_t fixed_bytes() { return sizeof(StepShared) + TW + 2 * FACB; }
     // per thread: W^t of the two gauge passes; per line: A, B, W^-n of both
-    static size_t smem(int C) {
-        return fixed_bytes() + (size_t)NBUF * C * L::LS * sizeof(cx<T>) + (size_t)C * P * 32 +
+    static size_t smem(int) {
+        return fixed_bytes() + (size_t)NBUF * C * LS * sizeof(cx<T>) + (size_t)C * P * 32 +
                (size_t)C * 96;
     }
 };
@@ -200,7 +205,7 @@ __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigne
 template <typename T, int N, int RA, int RB, int RC, int P, bool TAB, bool REAL, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     k_step2d(const __grid_constant__ StepArgs s) {
-    using S_ = StepShape<T, N, RA, RB, RC, P>;
+    using S_ = StepShape<T, N, RA, RB, RC, P, MAXT / P>;
     using L = typename S_::L;
     using Fac = std::conditional_t<std::is_same<T, float>::value, float2, double2>;
     constexpr int E = S_::E;
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     Fac* ky_s = vx_s + (S_::FAC ? N : 0);
     p += 2 * S_::FACB;
     cx<T>* xch = reinterpret_cast<cx<T>*>(p);
-    p += (size_t)S_::NBUF * C * L::LS * sizeof(cx<T>);
+    p += (size_t)S_::NBUF * C * S_::LS * sizeof(cx<T>);
     cx<double>* gt_s = reinterpret_cast<cx<double>*>(p);  // [2][threads]
     cx<double>* gl_s = gt_s + 2 * nthreads;               // [2][C][3]
 
@@ -297,8 +302,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
         // (the mask changes nothing: it lets the compiler fold the exchange offsets)
         const int t = (colpass ? tc : tr) & (P - 1);
         const int c = colpass ? cc : cr;
-        cx<T>* sl = xch + c * L::LS;
-        cx<T>* other = sl + (S_::NBUF - 1) * C * L::LS;
+        cx<T>* sl = xch + c * S_::LS;
+        cx<T>* other = sl + (S_::NBUF - 1) * C * S_::LS;
         const int base = colpass ? col : row * N, stride = colpass ? N : 1;
         auto sync = [&] {
             if constexpr (P <= 32) {
@@ -496,7 +501,7 @@ const StepKernel* step_table_f32(int* count);
 const StepKernel* step_table_f64(int* count);
 
 #define GPUE_STEP(T, N, RA, RB, RC, P, C, MINB)                                              \
-    StepKernel{N, RA, RB, RC, P, C, &StepShape<T, N, RA, RB, RC, P>::smem,                   \
+    StepKernel{N, RA, RB, RC, P, C, &StepShape<T, N, RA, RB, RC, P, C>::smem,                 \
                {{(const void*)&k_step2d<T, N, RA, RB, RC, P, false, false, C * P, MINB>,           \
                  (const void*)&k_step2d<T, N, RA, RB, RC, P, false, true, C * P, MINB>},           \
                 {(const void*)&k_step2d<T, N, RA, RB, RC, P, true, false, C * P, MINB>,            \
