@@ -26,7 +26,7 @@
 // point-steps/s of the multi-size line-pass kernel and here: 128 of 128^2 2.0e10
 // -> 5.6e10, 64 of 192^2 1.75e10 -> 5.4e10, 32 of 256^2 1.9e10 -> 4.7e10, 24 of
 // 512^2 1.8e10 -> 2.8e10 (7 clusters of 16 at a time), 16 of 384^2 1.4e10 ->
-// 2.2e10; complex128 32 of 128^2 1.4e10 -> 2.9e10.
+// 2.2e10; complex128 32 of 128^2 1.4e10 -> 3.1e10.
 //
 // Shared memory per CTA: the rows at a padded stride, which double as the
 // exchange buffer of their own transforms; an exchange buffer for the columns
@@ -64,9 +64,13 @@ template <typename T, int N, int RA, int RB, int RC, int P>
 struct ClusterShape {
     using L = LineFFT<T, N, RA, RB, P, RC>;
     static constexpr int E = L::E;
-    static constexpr int THREADS = N * P < kClusterThreads ? N * P : kClusterThreads;
+    // (256^2 complex128: 16 lines of 16 threads, so that clusters of 8 hold it
+    // with one exchange per transform: 8 solves 30.6 us per step; 8 4 8 with 512
+    // threads needs clusters of 16, 40.8)
+    static constexpr int MOST = sizeof(T) == 8 && N == 256 ? 256 : kClusterThreads;
+    static constexpr int THREADS = N * P < MOST ? N * P : MOST;
     static constexpr int LPR = THREADS / P;  // lines in flight
-    static constexpr int PHYS = smem_phys(N - 1) + 1;
+    static constexpr int PHYS = L::phys(N - 1) + 1;
     // row stride: lines of 8 threads share a half-warp, so offset them by half
     // a bank row
     static constexpr int XS = (PHYS + 15) / 16 * 16 + (P == 8 ? 8 : 0);
@@ -151,7 +155,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
     const cx<T>* in = static_cast<const cx<T>*>(a.in);
     for (int i = tid; i < mine * N; i += S_::THREADS) {
         const int r = i / N, x = i % N;
-        X[r * S_::XS + smem_phys(x)] = in[(size_t)(first + r) * N + x];
+        X[r * S_::XS + L::phys(x)] = in[(size_t)(first + r) * N + x];
     }
     __syncthreads();
     cluster_arrive();
@@ -199,7 +203,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
             auto remote = [&](int e) {
                 const unsigned y = (unsigned)L::index(t, e);
                 const unsigned q = __umulhi(y, Rmul);
-                return dsmem_map(xbase + ((y - q * R) * S_::XS + smem_phys(g)) * sizeof(cx<T>), q);
+                return dsmem_map(xbase + ((y - q * R) * S_::XS + L::phys(g)) * sizeof(cx<T>), q);
             };
             cx<T> v[E];
             if (colpass) {
@@ -207,7 +211,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
                 for (int e = 0; e < E; ++e) v[e] = dsmem_load<T>(remote(e));
             } else {
 #pragma unroll
-                for (int e = 0; e < E; ++e) v[e] = sl[smem_phys(L::index(t, e))];
+                for (int e = 0; e < E; ++e) v[e] = sl[L::phys(L::index(t, e))];
                 sync();  // the row is read before its exchanges write it
             }
             KSum acc{0.0, 0.0};
@@ -279,7 +283,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
                     for (int e = 0; e < E; ++e) dsmem_store<T>(remote(e), v[e]);
                 } else {
 #pragma unroll
-                    for (int e = 0; e < E; ++e) sl[smem_phys(L::index(t, e))] = v[e];
+                    for (int e = 0; e < E; ++e) sl[L::phys(L::index(t, e))] = v[e];
                 }
             }
             if (norm) {
@@ -322,7 +326,7 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
     cx<T>* out = static_cast<cx<T>*>(a.out);
     for (int i = tid; i < mine * N; i += S_::THREADS) {
         const int r = i / N, x = i % N;
-        out[(size_t)(first + r) * N + x] = X[r * S_::XS + smem_phys(x)];
+        out[(size_t)(first + r) * N + x] = X[r * S_::XS + L::phys(x)];
     }
     if (rank == 0 && tid == 0) {
         *s.scal_norm = sh->scale;

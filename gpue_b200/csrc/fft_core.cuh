@@ -298,7 +298,14 @@ struct LineFFT {
     static_assert((N / RA) % P == 0, "threads must divide the butterflies of the outer stages");
     static_assert(NS == 2 || (N / RB) % P == 0, "threads must divide the middle stages");
     static_assert(NS < 4 || (N / RC) % P == 0, "threads must divide the middle stages");
-    // smem line strides in complex elements: one pad per 16, rounded to 16, plus
+    // Element i of a line in shared memory: padded so that the first exchange,
+    // which writes RA elements apart per thread, spreads over the banks (a
+    // complex128 row of banks is 8 elements: one pad per 8 for RA = 4 and 8; per
+    // step 128^3 complex128 87 -> 77 us, 192^3 264 -> 248, 256^2 9.7 -> 9.2)
+    static constexpr int PADS = sizeof(T) == 8 && RA < 16 ? 3 : 4;
+    __host__ __device__ static constexpr int phys(int i) { return i + (i >> PADS); }
+
+    // smem line strides in complex elements: the padded length, rounded to 16, plus
     // an offset that puts the lines a warp touches at once on distinct banks.  A
     // shared-memory access is served 16 lanes (complex64) or 8 (complex128) at a
     // time.  Rows (LS): lanes are a line's threads, so only complex64 lines of 8
@@ -307,7 +314,7 @@ struct LineFFT {
     // threads, so the lines lie that many elements apart.  With one offset of 4 for
     // all, complex128 columns of 8-thread lines met 4 to a bank: per step on B200
     // 96^3 complex128 56 -> 47 us, rotating 82 -> 64, 160^3 complex64 113 -> 103.
-    static constexpr int kPad16 = ((smem_phys(N - 1) + 1 + 15) / 16) * 16;
+    static constexpr int kPad16 = ((phys(N - 1) + 1 + 15) / 16) * 16;
     static constexpr int LS = kPad16 + (sizeof(T) == 4 && P == 8 ? 8 : 4);
     static constexpr int LSC =
         kPad16 + (sizeof(T) == 4 ? (P >= 16 ? P / 8 : 1) : (P >= 32 ? P / 16 : 1));
@@ -463,7 +470,7 @@ struct LineFFT {
             const int j = t + P * q;
             const int base = (j / Ns) * Ns * R + (j % Ns);
 #pragma unroll
-            for (int r = 0; r < R; ++r) sl[smem_phys(base + r * Ns)] = v[q * R + r];
+            for (int r = 0; r < R; ++r) sl[phys(base + r * Ns)] = v[q * R + r];
         }
         sync();
         constexpr int R2 = radix(S + 1);
@@ -472,7 +479,7 @@ struct LineFFT {
         for (int q = 0; q < G2; ++q) {
             const int j = t + P * q;
 #pragma unroll
-            for (int r = 0; r < R2; ++r) v[q * R2 + r] = sl[smem_phys(j + r * (N / R2))];
+            for (int r = 0; r < R2; ++r) v[q * R2 + r] = sl[phys(j + r * (N / R2))];
         }
         sync();
     }
@@ -492,7 +499,7 @@ struct LineFFT {
             const int j = t + P * q;
             const int base = (j / Ns) * Ns * R + (j % Ns);
 #pragma unroll
-            for (int r = 0; r < R; ++r) sl[smem_phys(base + r * Ns)] = v[q * R + r];
+            for (int r = 0; r < R; ++r) sl[phys(base + r * Ns)] = v[q * R + r];
         }
         sync();
         constexpr int R2 = radix(S + 1);
@@ -501,7 +508,7 @@ struct LineFFT {
         for (int q = 0; q < G2; ++q) {
             const int j = t + P * q;
 #pragma unroll
-            for (int r = 0; r < R2; ++r) v[q * R2 + r] = sl[smem_phys(j + r * (N / R2))];
+            for (int r = 0; r < R2; ++r) v[q * R2 + r] = sl[phys(j + r * (N / R2))];
         }
         cx<T>* const w = sl;
         sl = other;
