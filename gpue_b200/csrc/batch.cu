@@ -88,6 +88,29 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
            c->xy[prec].k && c->zpass[prec].k && plane_ok(c, prec);
 }
 
+// 2D solves that run on the grid-wide stepper, one after another.  Complex64 up
+// to 512^2: those too large for a cluster to step quickly alone, 512^2 and 384^2
+// with the gauge (one of 512^2 per step as line passes, as a cluster of 16 and as
+// a grid: 30, 55 and 12 us; rotating 48, 102 and 18; 24 of them 342, 220 and 287,
+// so many alike would be faster on clusters).  From 768: line passes in groups
+// and grid, 8 of 768^2 complex64 218 and 165 us (complex128 306 and 206), 8 of 1024^2 270 and 197, one 41
+// and 25, 4 of 1024^2 complex128 232 and 141.  In between the groups are faster
+// as soon as several share them: 8 of 384^2 complex128 70 and 112, 8 of 640^2 198
+// and 208, 24 of 640^2 complex64 426 and 468, though one alone is not (384^2
+// complex128 56 and 14).  The choice is the solve's own, never the mix's, so a
+// result does not depend on its company.
+bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
+    const char* env = std::getenv("GPUE_BATCH_MEGA");
+    if (env && env[0] == '0') return false;
+    if (c->dim != 2 || !c->step[prec].k || c->ext || c->time_dep || c->line_plan) return false;
+    if (c->ax[0].n < 768) {
+        if (prec != GPUE_PREC_FP32 || c->ax[0].n > 512) return false;
+        const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
+        if (c->N * (gauge ? 2 : 1) < (1L << 18)) return false;
+    }
+    return step_ready(c, prec, gstate);
+}
+
 // Cluster sizes of a run's 2D solves (0: not on the cluster stepper).  A solve
 // starts at the smallest cluster that holds its field; while the device has
 // room, the one with most points per CTA doubles, so a mix finishes together
@@ -111,6 +134,7 @@ std::vector<int> cluster_sizes(const BatchRun& r) {
         gpue_ctx* c = r.ctx[i];
         const ClusterKernel* k = c->cluster[c->prec].k;
         if (!k || c->ext || c->time_dep || c->line_plan) continue;
+        if (grid_eligible(c, c->prec, r.gstate)) continue;
         int max_smem = 0;
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
         int s = 1;
@@ -151,9 +175,10 @@ void group_solves(BatchRun& r, int probe) {
         gpue_ctx* c = r.ctx[i];
         const int off = r.offset[i];
         const bool tile = tile_eligible(c, c->prec);
+        const bool grid = !cs[i] && grid_eligible(c, c->prec, r.gstate);
         const std::string sig =
             std::to_string((int)r.guard[i]) + "/" + (tile ? "tile/" : "") +
-            (cs[i] ? "cluster" + std::to_string(cs[i]) + "/" : "") +
+            (cs[i] ? "cluster" + std::to_string(cs[i]) + "/" : "") + (grid ? "grid/" : "") +
             pass_signature(c, c->prec,
                            solve_passes(c, off, off + probe, r.gstate, r.guard[i], r.scale_step0,
                                         tile));
@@ -165,7 +190,8 @@ void group_solves(BatchRun& r, int probe) {
             g.guard = r.guard[i];
             g.tile = tile;
             g.cluster = cs[i];
-            g.mega = !tile && !g.cluster && mega_eligible(c, c->prec);
+            g.grid = grid;
+            g.mega = !tile && !g.cluster && !grid && mega_eligible(c, c->prec);
             r.groups.push_back(g);
         }
         r.groups[it->second].members.push_back((int)i);
@@ -350,6 +376,35 @@ static gpue_status plan_cluster_launch(const BatchRun& r, const BGroup& g, int s
     return GPUE_OK;
 }
 
+// The steps [s0, s1) of a grid group: one cooperative launch per solve (per
+// kStepChunk steps) on the group's lane.
+static gpue_status plan_grid_launches(const BatchRun& r, const BGroup& g, int s0, int s1,
+                                      std::vector<LaunchOp>& ops, long& launches,
+                                      std::string& err) {
+    for (int m : g.members) {
+        gpue_ctx* c = r.ctx[m];
+        for (int a0 = s0; a0 < s1; a0 += kStepChunk) {
+            const int i0 = r.offset[m] + a0, n = std::min(kStepChunk, s1 - a0);
+            const std::vector<StepPass> walk =
+                step_walk(c, i0, n, r.gstate, r.gstate == 0 && (i0 > 0 || r.scale_step0),
+                          r.guard[m] ? 1 : 0);
+            auto s = std::make_shared<StepArgs>();
+            gpue_status st = step_args(c, g.prec, r.gstate, walk, *s);
+            if (st) {
+                err = c->err;
+                return st;
+            }
+            const StepCfg sc = c->step[g.prec];
+            const int gstate = r.gstate;
+            ops.push_back([=](cudaStream_t stream) {
+                launch_grid_steps(sc, false, gstate, *s, stream);
+            });
+            launches++;
+        }
+    }
+    return GPUE_OK;
+}
+
 gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink& sink,
                          SegPlan& sp, std::string& err) {
     sp.lanes.assign(r.groups.size(), {});
@@ -368,6 +423,11 @@ gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink&
         const int n = (int)g.members.size();
         gpue_ctx* c0 = r.ctx[g.members[0]];
         std::vector<std::vector<LPass>> lists(n);
+        if (g.grid) {
+            gpue_status st = plan_grid_launches(r, g, s0, s1, out_ops, sp.launches, err);
+            if (st) return st;
+            if (!check) continue;
+        }
         if (g.cluster) {
             gpue_status st = plan_cluster_launch(r, g, s0, s1, sink, out_ops, err);
             if (st) return st;
@@ -377,7 +437,7 @@ gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink&
         for (int k = 0; k < n; ++k) {
             const int m = g.members[k];
             gpue_ctx* c = r.ctx[m];
-            if (!g.mega && !g.cluster)
+            if (!g.mega && !g.cluster && !g.grid)
                 lists[k] = solve_passes(c, r.offset[m] + s0, r.offset[m] + s1, r.gstate,
                                         r.guard[m], r.scale_step0, g.tile);
             if (check)
@@ -806,7 +866,8 @@ gpue_status gpue_batch_evolve(gpue_batch* b, int32_t gstate, const gpue_batch_op
         std::snprintf(tb, sizeof tb, "%a:", run.thr);
         k += tb;
         for (const BGroup& g : run.groups) {
-            k += "{" + std::to_string(g.guard) + "/" + std::to_string(g.cluster) + "/" +
+            k += "{" + std::to_string(g.guard) + "/" + std::to_string(g.cluster) +
+                 (g.grid ? "g/" : "/") +
                  pass_signature(run.ctx[g.members[0]], g.prec,
                                 solve_passes(run.ctx[g.members[0]], 0, 3, gstate, g.guard,
                                              false, g.tile)) + "}";

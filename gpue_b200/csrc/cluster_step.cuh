@@ -24,9 +24,10 @@
 // threads at 64 registers were no faster: 256^2 45 -> 50 us); the rest is the
 // column groups' barriers and remote loads.  Batched complex64 solves on B200,
 // point-steps/s of the multi-size line-pass kernel and here: 128 of 128^2 2.0e10
-// -> 5.6e10, 64 of 192^2 1.75e10 -> 5.4e10, 32 of 256^2 1.9e10 -> 4.7e10, 24 of
-// 512^2 1.8e10 -> 2.8e10 (7 clusters of 16 at a time), 16 of 384^2 1.4e10 ->
-// 2.2e10; complex128 32 of 128^2 1.4e10 -> 3.1e10.
+// -> 5.6e10, 64 of 192^2 1.75e10 -> 5.4e10, 32 of 256^2 1.9e10 -> 4.7e10, 16 of
+// 384^2 1.4e10 -> 2.2e10 (7 clusters of 16 at a time); complex128 32 of 128^2
+// 1.4e10 -> 3.1e10.  A lone solve gets 16 SMs at most: complex128 256^2 39 -> 19 us per
+// step, but complex64 512^2 30 -> 55, so that one runs on the grid (batch.cu).
 //
 // Shared memory per CTA: the rows at a padded stride, which double as the
 // exchange buffer of their own transforms; an exchange buffer for the columns

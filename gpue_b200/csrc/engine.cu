@@ -515,7 +515,7 @@ gpue_status plan_step(gpue_ctx* c, int prec) {
 // The stepper kernel of this context's fields and time kind, if its whole grid
 // is resident at once (every CTA waits for all others).  Asked when steps are
 // first run, so a context loads only the kernel it uses.
-static bool step_ready(gpue_ctx* c, int prec, int gstate) {
+bool step_ready(gpue_ctx* c, int prec, int gstate) {
     StepCfg& sc = c->step[prec];
     int& r = sc.ready[c->ext ? 1 : 0][gstate ? 1 : 0];
     if (r == 0) {
@@ -1040,9 +1040,6 @@ gpue_status enqueue_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, boo
     return GPUE_OK;
 }
 
-// Most steps one resident launch holds (at most 6 passes a step)
-constexpr int kStepChunk = kStepMaxSeq / 6;
-
 namespace {
 
 // The passes of n steps from i0 as the resident stepper walks them.
@@ -1204,17 +1201,10 @@ bool step_ok(gpue_ctx* c, int prec, int gstate) {
     return cluster_ok(c, prec, gstate) || step_ready(c, prec, gstate);
 }
 
-// Steps [i0, i1) as one launch: a cluster, or a cooperative grid.
-gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool scale_first,
-                         int guard) {
-    const GraphKey key{prec, gstate, i0 % 4, i1 - i0, scale_first ? 1 : 0, 0, guard, 0};
-    auto it = c->step_seq.find(key);
-    if (it == c->step_seq.end())
-        it = c->step_seq.emplace(key, step_walk(c, i0, i1 - i0, gstate, scale_first, guard)).first;
-    const std::vector<StepPass>& walk = it->second;
+gpue_status step_args(gpue_ctx* c, int prec, int gstate, const std::vector<StepPass>& walk,
+                      StepArgs& s) {
     if (walk.size() > (size_t)kStepMaxSeq)
         return fail(c, GPUE_ERR_STATE, "a resident launch holds at most %d passes", kStepMaxSeq);
-    StepArgs s;
     gpue_status st = stepper_consts(c, prec, gstate, s.a, s.gauge_ang);
     if (st) return st;
     s.sync = c->counters + kCtrStep;
@@ -1226,6 +1216,37 @@ gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool
     s.err = c->dflags + 3;
     s.nseq = (int)walk.size();
     std::copy(walk.begin(), walk.end(), s.seq);
+    return GPUE_OK;
+}
+
+cudaError_t launch_grid_steps(const StepCfg& sc, bool tables, int gstate, const StepArgs& s,
+                              cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sc.blocks);
+    cfg.blockDim = dim3(sc.threads);
+    cfg.dynamicSmemBytes = sc.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    void* args[] = {const_cast<StepArgs*>(&s)};
+    return cudaLaunchKernelExC(&cfg, sc.k->fn[tables ? 1 : 0][gstate ? 1 : 0], args);
+}
+
+// Steps [i0, i1) as one launch: a cluster, or a cooperative grid.
+gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool scale_first,
+                         int guard) {
+    const GraphKey key{prec, gstate, i0 % 4, i1 - i0, scale_first ? 1 : 0, 0, guard, 0};
+    auto it = c->step_seq.find(key);
+    if (it == c->step_seq.end())
+        it = c->step_seq.emplace(key, step_walk(c, i0, i1 - i0, gstate, scale_first, guard)).first;
+    const std::vector<StepPass>& walk = it->second;
+    StepArgs s;
+    gpue_status st = step_args(c, prec, gstate, walk, s);
+    if (st) return st;
+    s.a.active = nullptr;  // a single solve always runs
     void* args[] = {&s};
     const ClusterCfg& cc = c->cluster[prec];
     if (cluster_ok(c, prec, gstate)) {
@@ -1233,18 +1254,7 @@ gpue_status launch_steps(gpue_ctx* c, int prec, int i0, int i1, int gstate, bool
         c->launches++;
         return GPUE_OK;
     }
-    const StepCfg& sc = c->step[prec];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sc.blocks);
-    cfg.blockDim = dim3(sc.threads);
-    cfg.dynamicSmemBytes = sc.smem;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelExC(&cfg, sc.k->fn[c->ext ? 1 : 0][gstate ? 1 : 0], args));
+    CK(launch_grid_steps(c->step[prec], c->ext, gstate, s, c->stream));
     c->launches++;
     return GPUE_OK;
 }

@@ -322,6 +322,15 @@ cudaError_t launch_cluster(const ClusterKernel* k, const void* fn, int cs, int c
 // The walk of a context's steps [i0, i0 + n) (stepper.cuh).
 std::vector<StepPass> step_walk(gpue_ctx* c, int i0, int n, int gstate, bool scale_first,
                                 int guard);
+// Most steps one resident launch holds (at most 6 passes a step)
+constexpr int kStepChunk = kStepMaxSeq / 6;
+// Whether the grid stepper's kernel for this time kind can run (stepper.cuh).
+bool step_ready(gpue_ctx* c, int prec, int gstate);
+// The arguments of a stepper launch that walks `walk`, and that launch.
+gpue_status step_args(gpue_ctx* c, int prec, int gstate, const std::vector<StepPass>& walk,
+                      StepArgs& s);
+cudaError_t launch_grid_steps(const StepCfg& sc, bool tables, int gstate, const StepArgs& s,
+                              cudaStream_t stream);
 // The rotation gauge's angles per momentum index and unit position, and the
 // per-call constants of a stepper launch.
 gpue_status stepper_consts(gpue_ctx* c, int prec, int gstate, PassArgs& a, double (&ang)[2]);

@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
 
     const PassArgs& a = s.a;
     const int ncta = (int)gridDim.x, rank = (int)blockIdx.x;
+    // a converged solve of a batched run: every CTA leaves before the first barrier
+    if (a.active && *a.active == 0) return;
 
     // shared memory: StepShared | stage twiddles | V/2 x, K y factors |
     // exchange | W^t of both gauge passes | their line constants
