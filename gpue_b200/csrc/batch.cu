@@ -92,13 +92,13 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
 // to 512^2: those too large for a cluster to step quickly alone, 512^2 and 384^2
 // with the gauge (one of 512^2 per step as line passes, as a cluster of 16 and as
 // a grid: 30, 55 and 12 us; rotating 48, 102 and 18; 24 of them 342, 220 and 287,
-// so many alike would be faster on clusters).  From 768: line passes in groups
-// and grid, 8 of 768^2 complex64 218 and 165 us (complex128 306 and 206), 8 of 1024^2 270 and 197, one 41
-// and 25, 4 of 1024^2 complex128 232 and 141.  In between the groups are faster
-// as soon as several share them: 8 of 384^2 complex128 70 and 112, 8 of 640^2 198
-// and 208, 24 of 640^2 complex64 426 and 468, though one alone is not (384^2
-// complex128 56 and 14).  The choice is the solve's own, never the mix's, so a
-// result does not depend on its company.
+// so many alike would be faster on clusters).  From 768 on, line passes in
+// groups and the grid: 8 of 768^2 complex64 218 and 165 us, complex128 306 and
+// 206, 8 of 1024^2 complex64 270 and 197, one 41 and 25, 4 of 1024^2 complex128
+// 232 and 141.  In between the groups are faster as soon as several share them,
+// 8 of 384^2 complex128 70 and 112, 8 of 640^2 198 and 208, 24 of 640^2 complex64
+// 426 and 468, though one alone is not (384^2 complex128 56 and 14).  The choice
+// is the solve's own, never the mix's, so a result does not depend on its company.
 bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
     const char* env = std::getenv("GPUE_BATCH_MEGA");
     if (env && env[0] == '0') return false;
