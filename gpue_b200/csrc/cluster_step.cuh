@@ -257,12 +257,6 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
                     case OP_GAUGE: {
                         const double ang =
                             (colpass ? s.gauge_ang[1] : s.gauge_ang[0]) * a.pos[colpass ? 0 : 1][g];
-                        if constexpr (std::is_same<T, float>::value) {
-                            if (gauge_small(ang, N)) {
-                                op_gauge_f32<L>(v, t, ang, gstate, a.gscale);
-                                break;
-                            }
-                        }
                         op_gauge<T, L>(v, gauge_consts<L>(t, ang, gstate, a.gscale), gstate);
                         break;
                     }

@@ -524,7 +524,9 @@ __device__ __forceinline__ void op_norm_f32(const cx<float> (&v)[E], KSum& acc) 
 // frequency of index k (m = k - n for k >= n/2).  It is geometric in k: the
 // factor of k = t + P q + r n/RA is W^t A^q B^r, times W^-n for r >= RA/2
 // (t + P q < n/RA, so k >= n/2 exactly there), with W = w(dp), A = W^P,
-// B = W^(n/RA), all formed in FP64.  ang1 is the angle per unit m.
+// B = W^(n/RA), all formed and applied in FP64, for complex64 too: an FP32 series
+// left served rotating solves 6 to 12 %
+// further from the FP64 result.  ang1 is the angle per unit m.
 
 struct GaugeConsts {
     cx<double> wt, wa, wb, wn;  // W^t gscale, W^P, W^(n/RA), W^-n
@@ -571,41 +573,6 @@ __device__ __forceinline__ void op_gauge(cx<T> (&v)[L::E], const GaugeConsts& g,
             }
             aq = cmul(aq, g.wa);
         }
-    }
-}
-
-// Complex64: the whole line's angles below 1/16, where the factor minus 1 comes
-// from its FP32 Taylor series (relative truncation below 2^-24) and is applied
-// as psi + d*psi, as the other complex64 factors are.  The FP64 chain costs a
-// conversion of every component each way, which run at a fraction of the FP32
-// rate: on the 1024^2 rotating case it was a third of the pass's issue slots.
-__device__ __forceinline__ bool gauge_small(double ang1, int n) {
-    return fabs(ang1) * (0.5 * n) < 0.0625;
-}
-template <class L>
-__device__ __forceinline__ void op_gauge_f32(cx<float> (&v)[L::E], int t, double ang1, int gstate,
-                                             double gscale) {
-    constexpr int N = L::N, RA = L::radix(0);
-    // the angle per unit m and the scale as hi + lo floats: the angle is then
-    // rounded once per element, and the rounded part of the scale (which would
-    // be a systematic error of every step) enters the factor
-    const float ch = (float)ang1, cl = (float)(ang1 - (double)ch), tf = (float)t;
-    const float s = (float)gscale;
-    const float eps = (float)((gscale - (double)s) * (double)N);  // gscale = 1/N
-#pragma unroll
-    for (int e = 0; e < L::E; ++e) {
-        const int r = e % RA;
-        const float m = tf + (float)(L::P * (e / RA) + r * (N / RA) - (r >= RA / 2 ? N : 0));
-        const float p = fmaf(m, ch, m * cl);
-        cx<float> w;
-        if (gstate == 0) {
-            w = dapply_re(v[e], nl_decay_delta(p) + eps);
-        } else {
-            float2 d = nl_phase_delta(p);
-            d.x += eps;
-            w = dapply(v[e], d);
-        }
-        v[e] = {w.x * s, w.y * s};
     }
 }
 
@@ -827,12 +794,6 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     const int src = a.gauge_src;
                     const int sidx = (src == 0) ? xi : (src == 1) ? yi : zi;
                     const double ang1 = a.gauge_coef * a.pos[src][sidx] * a.gauge_dt * a.dmom;
-                    if constexpr (std::is_same<T, float>::value) {
-                        if (gauge_small(ang1, N)) {
-                            op_gauge_f32<L>(v, t, ang1, a.gstate, a.gscale);
-                            break;
-                        }
-                    }
                     op_gauge<T, L>(v, gauge_consts<L>(t, ang1, a.gstate, a.gscale), a.gstate);
                     break;
                 }

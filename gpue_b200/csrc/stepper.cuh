@@ -272,15 +272,10 @@ __global__ void __launch_bounds__(MAXT, MINB)
     // the rotation gauge's angles per momentum index along the row and column
     const double ang[2] = {s.gauge_ang[0] * a.pos[1][row_ok ? row : 0],
                            s.gauge_ang[1] * a.pos[0][col_ok ? col : 0]};
-    bool gsm[2] = {false, false};
     if constexpr (!TAB) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             if (s.gauge_ang[g] == 0.0) continue;
-            if constexpr (std::is_same<T, float>::value) {
-                gsm[g] = gauge_small(ang[g], N);
-                if (gsm[g]) continue;
-            }
             const int t = g ? tc : tr, c = g ? cc : cr;
             const GaugeConsts gc = gauge_consts<L>(t, ang[g], gstate, a.gscale);
             gt_s[g * nthreads + tid] = gc.wt;
@@ -411,13 +406,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
                         op_gauge<T, L>(v, gauge_consts<L>(t, ang[g], gstate, a.gscale),
                                        gstate);
                     } else {
-                        if constexpr (std::is_same<T, float>::value) {
-                            if (colpass ? gsm[1] : gsm[0]) {
-                                op_gauge_f32<L>(v, t, colpass ? ang[1] : ang[0], gstate,
-                                                a.gscale);
-                                break;
-                            }
-                        }
                         const cx<double>* gl = gl_s + (g * C + c) * 3;
                         op_gauge<T, L>(v, GaugeConsts{gt_s[g * nthreads + tid], gl[0], gl[1], gl[2]},
                                        gstate);

@@ -505,14 +505,7 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS,
                         L::template forward<true>(v, t, sl, twp, sync);
                         const double ang =
                             a.gauge_coef * a.pos[YX ? 1 : 0][line] * a.gauge_dt * a.dmom;
-                        bool small = false;
-                        if constexpr (F32) {
-                            small = gauge_small(ang, N);
-                            if (small) op_gauge_f32<L>(v, t, ang, a.gstate, a.gscale);
-                        }
-                        if (!small)
-                            op_gauge<T, L>(v, gauge_consts<L>(t, ang, a.gstate, a.gscale),
-                                           a.gstate);
+                        op_gauge<T, L>(v, gauge_consts<L>(t, ang, a.gstate, a.gscale), a.gstate);
                         __syncwarp();
                         L::template forward<true, true>(v, t, sl, twp, sync);
                     }
