@@ -524,9 +524,9 @@ __device__ __forceinline__ void op_norm_f32(const cx<float> (&v)[E], KSum& acc) 
 // frequency of index k (m = k - n for k >= n/2).  It is geometric in k: the
 // factor of k = t + P q + r n/RA is W^t A^q B^r, times W^-n for r >= RA/2
 // (t + P q < n/RA, so k >= n/2 exactly there), with W = w(dp), A = W^P,
-// B = W^(n/RA), all formed and applied in FP64, for complex64 too: an FP32 series
-// left served rotating solves 6 to 12 %
-// further from the FP64 result.  ang1 is the angle per unit m.
+// B = W^(n/RA), all formed and applied in FP64, for complex64 too (with
+// an FP32 series here, served rotating solves were 6 to 12 % further from the
+// FP64 result).  ang1 is the angle per unit m.
 
 struct GaugeConsts {
     cx<double> wt, wa, wb, wn;  // W^t gscale, W^P, W^(n/RA), W^-n
