@@ -126,7 +126,7 @@ std::vector<int> cluster_sizes(const BatchRun& r) {
     if (env && env[0] == '0') return cs;
     auto share = [&](size_t i, int s) {  // of the device; > 1: such a cluster does not fit
         const ClusterKernel* k = r.ctx[i]->cluster[r.ctx[i]->prec].k;
-        const int m = clusters_resident(k, k->many[r.gstate], s);
+        const int m = clusters_resident(r.ctx[i]->device, k, k->many[r.gstate], s);
         return m > 0 ? 1.0 / m : 2.0;
     };
     double total = 0;

@@ -1124,13 +1124,13 @@ cudaError_t launch_cluster(const ClusterKernel* k, const void* fn, int cs, int c
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-int clusters_resident(const ClusterKernel* k, const void* fn, int cs) {
-    // asked once per kernel and size: the answer is the device's and does not
-    // change (every device of a node is of one kind)
+int clusters_resident(int device, const ClusterKernel* k, const void* fn, int cs) {
+    // asked once per device, kernel and size: the answer does not change, and
+    // the attributes set below hold on the device they were set on only
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> known;
+    static std::map<std::tuple<int, const void*, int>, int> known;
     std::lock_guard<std::mutex> lk(mu);
-    auto it = known.find({fn, cs});
+    auto it = known.find({device, fn, cs});
     if (it != known.end()) return it->second;
     const int smem = (int)k->smem(cs);
     int n = 0;
@@ -1160,7 +1160,7 @@ int clusters_resident(const ClusterKernel* k, const void* fn, int cs) {
         cudaGetLastError();  // not an error of the call that asks
         n = 0;
     }
-    known[{fn, cs}] = n;
+    known[{device, fn, cs}] = n;
     return n;
 }
 
@@ -1190,7 +1190,7 @@ static bool cluster_ok(gpue_ctx* c, int prec, int gstate) {
     if (!cc.k || c->ext) return false;
     if (c->ax[0].n > kClusterAlone) return false;
     int& r = cc.ready[gstate ? 1 : 0];
-    if (r == 0) r = clusters_resident(cc.k, cc.k->one[gstate ? 1 : 0], cc.cs) > 0 ? 1 : -1;
+    if (r == 0) r = clusters_resident(c->device, cc.k, cc.k->one[gstate ? 1 : 0], cc.cs) > 0 ? 1 : -1;
     return r > 0;
 }
 

@@ -16,6 +16,7 @@
 #include <mutex>
 #include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/gpue_b200.h"
@@ -312,10 +313,10 @@ gpue_status plan_step(gpue_ctx* c, int prec);
 // Plans the 2D cluster stepper of precision prec (lengths whose field fits a
 // cluster's shared memory); leaves it off otherwise.
 gpue_status plan_cluster(gpue_ctx* c, int prec);
-// How many clusters of cs CTAs of kernel fn the device holds at once (0: none
-// fits); prepares fn for its launches.  Asked before a kernel's first launch,
-// so only kernels in use are loaded.
-int clusters_resident(const ClusterKernel* k, const void* fn, int cs);
+// How many clusters of cs CTAs of kernel fn the device (the current one) holds
+// at once (0: none fits); prepares fn for its launches there.  Asked before a
+// kernel's first launch on a device, so only kernels in use are loaded.
+int clusters_resident(int device, const ClusterKernel* k, const void* fn, int cs);
 // Launches `clusters` clusters of cs CTAs.
 cudaError_t launch_cluster(const ClusterKernel* k, const void* fn, int cs, int clusters,
                            cudaStream_t s, void** args);
