@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256, 2) k_observables(const ObsArgs o) {
 // solves still running.
 struct CheckArgs {
     double* scal;       // the solve's scalar slots
-    int* flags;         // [0] active, [1] steps done when it stopped, [2] checks
+    int* flags;         // [0] active, [1] steps done when it stopped, [2] checks, [3] a wait gave up
     double inv_n;       // 1/N
     double dV;
     int slot_ekin, slot_ereal, slot_eold, slot_e;
@@ -345,7 +345,7 @@ struct BatchOut {
     int active;
     int steps;
     int checks;
-    int pad;
+    int gave_up;  // a bounded wait of one of its passes ran out: the state is not valid
 };
 
 static __global__ void k_batch_gather(const CheckArgs* __restrict__ args, int n, BatchOut* out) {
@@ -355,7 +355,7 @@ static __global__ void k_batch_gather(const CheckArgs* __restrict__ args, int n,
         out[s].active = c.flags[0];
         out[s].steps = c.flags[1];
         out[s].checks = c.flags[2];
-        out[s].pad = 0;
+        out[s].gave_up = c.flags[3];
     }
 }
 

@@ -319,7 +319,6 @@ gpue_status plan_mega(const BatchRun& r, int prec, int s0, int s1, ArgSink& sink
     ma.args = static_cast<const PassArgs*>(dargs);
     ma.ticket = reinterpret_cast<unsigned long long*>(const_cast<void*>(dctr));
     ma.done = reinterpret_cast<int*>(const_cast<void*>(dctr)) + 2;
-    ma.err = c0->dflags + 3;
     const size_t ctr_bytes = zeros.size() * sizeof(int);
     void* ctr = const_cast<void*>(dctr);
     ops.push_back([=](cudaStream_t s) {
@@ -993,6 +992,7 @@ gpue_status gpue_batch_evolve(gpue_batch* b, int32_t gstate, const gpue_batch_op
     float ms = 0.f;
     BCK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
     double point_steps = 0;
+    std::string gave_up;  // solves whose state a wait that ran out has spoiled
     for (int i = 0; i < n; ++i) {
         gpue_ctx* c = b->ctx[i];
         const BatchOut& bo = b->h_outs[i];
@@ -1008,6 +1008,10 @@ gpue_status gpue_batch_evolve(gpue_batch* b, int32_t gstate, const gpue_batch_op
         if (gstate == 0) c->pending_scale = true;
         BCTX(c, apply_pending_scale(c, c->prec));
         if (guard_all[i]) BCTX(c, scale_state(c, c->prec, kGuard));
+        if (bo.gave_up) {
+            gave_up += (gave_up.empty() ? "" : ", ") + std::to_string(i);
+            BCK(cudaMemsetAsync(c->dflags + 3, 0, sizeof(int), c->stream));
+        }
     }
     for (int i = 0; i < n; ++i) BCK(cudaStreamSynchronize(b->ctx[i]->stream));
     if (stats) {
@@ -1016,6 +1020,9 @@ gpue_status gpue_batch_evolve(gpue_batch* b, int32_t gstate, const gpue_batch_op
         stats->graph_launches = glaunches;
         stats->point_steps = point_steps;
     }
+    if (!gave_up.empty())
+        return bfail(b, GPUE_ERR_TIMEOUT, "a pass of solve %s gave up waiting for its data",
+                     gave_up.c_str());
     return GPUE_OK;
 }
 

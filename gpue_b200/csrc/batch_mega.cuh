@@ -12,8 +12,8 @@
 // finished all its items (a per-instance completion counter).  Tickets are taken in order and
 // a tile only ever waits on tiles with smaller tickets, which CTAs that are
 // already running took, so the walk always progresses whatever the number of
-// resident CTAs; the wait is bounded all the same (a flag records a wait that
-// gave up, and the run reports GPUE_ERR_TIMEOUT).
+// resident CTAs; the wait is bounded all the same (the waiting solve's flag
+// records one that gave up, and the run reports GPUE_ERR_TIMEOUT).
 //
 // Every tile runs the line-pass body of its solve's length and axis (the same
 // code as the single-solve passes), with a fixed 256 threads per CTA: C =
@@ -47,7 +47,6 @@ struct MegaArgs {
     const PassArgs* args;
     unsigned long long* ticket;  // zero before the launch
     int* done;                   // [npass] finished items, zero before the launch
-    int* err;                    // set when a dependency wait gave up
 };
 
 constexpr unsigned kMegaWaitPolls = 1u << 24;

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kMegaThreads, 2) k_batch_mega(const MegaArgs m
                     unsigned polls = 0;
                     while (*d < need) {
                         if (++polls >= kMegaWaitPolls) {
-                            atomicExch(m.err, 1);
+                            atomicExch(m.args[m.passes[pi].args].err, 1);
                             break;
                         }
                         __nanosleep(64);

@@ -425,8 +425,9 @@ gpue_status issue_run(gpue_server* S, int gstate, Run& R, long& launches, std::s
 
 // A solve's result: final scaling, copy-out, result (to push).  `why` is
 // GPUE_OK for a solve that ran to its end, or the timeout / cancellation
-// status of one that leaves early (its state still goes to psi_out).  Its
-// context stays allocated (and counted against the budget) until release().
+// status of one that leaves early (its state still goes to psi_out, unless a
+// wait on the device gave up and left none).  Its context stays allocated (and
+// counted against the budget) until release().
 gpue_server_result finish(gpue_server* S, Solve& s, const BatchOut& bo, bool stopped,
                           gpue_status why = GPUE_OK) {
     gpue_ctx* c = s.c;
@@ -434,12 +435,12 @@ gpue_server_result finish(gpue_server* S, Solve& s, const BatchOut& bo, bool sto
     if (s.req.gstate == 0) c->pending_scale = true;
     st = apply_pending_scale(c, c->prec);
     if (!st && s.guard) st = scale_state(c, c->prec, kGuard);
-    if (!st && s.req.psi_out) st = gpue_get_wfc(c, s.req.psi_out, GPUE_MEM_HOST, GPUE_C128);
+    if (!st && s.req.psi_out && !bo.gave_up) st = gpue_get_wfc(c, s.req.psi_out, GPUE_MEM_HOST, GPUE_C128);
     if (!st && cudaStreamSynchronize(c->stream) != cudaSuccess) st = GPUE_ERR_CUDA;
     gpue_server_result r = make_result(s.req, st ? st : why, s.t_submit, s.t_admit, now_s(S));
     r.steps_done = stopped ? bo.steps : s.steps;
     r.early_stop = stopped ? 1 : 0;
-    r.energy = bo.checks > 0 ? bo.energy : NAN;
+    r.energy = bo.checks > 0 && !bo.gave_up ? bo.energy : NAN;
     {
         std::lock_guard<std::mutex> lk(S->mu);
         if (r.status == GPUE_ERR_TIMEOUT) S->st.timed_out++;
@@ -545,7 +546,9 @@ gpue_status tick_complete(gpue_server* S, long launches, std::string& err) {
             pts += (double)s.c->N * S->o.check_steps;
             const bool stopped = g == 0 && bo.active == 0;
             gpue_status why = GPUE_OK;
-            if (!stopped && s.steps < s.req.max_steps) {
+            if (bo.gave_up) {
+                why = GPUE_ERR_TIMEOUT;
+            } else if (!stopped && s.steps < s.req.max_steps) {
                 if (cancel.count(s.req.tag)) why = GPUE_ERR_CANCELLED;
                 else if (expired(s.req, s.t_submit, now)) why = GPUE_ERR_TIMEOUT;
             }

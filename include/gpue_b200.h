@@ -423,7 +423,9 @@ gpue_status gpue_batch_destroy(gpue_batch* batch);
 const char* gpue_batch_last_error(const gpue_batch* batch);
 /* Runs every solve from its current state; results[i] belongs to ctxs[i];
  * results and stats may be NULL.  Afterwards each context holds its final
- * state as if gpue_evolve had run it alone. */
+ * state as if gpue_evolve had run it alone.  GPUE_ERR_TIMEOUT when a bounded
+ * device wait of a solve gave up: the message of gpue_batch_last_error names
+ * the solves whose states are not valid then, the others are complete. */
 gpue_status gpue_batch_evolve(gpue_batch* batch, int32_t gstate, const gpue_batch_opts* opts,
                               gpue_batch_result* results, gpue_batch_stats* stats);
 
@@ -461,7 +463,9 @@ typedef struct gpue_request {
     double deadline_s;   /* 0: none; else the request fails with GPUE_ERR_TIMEOUT once this
                             many seconds have passed since its submission (checked while it
                             waits and after every tick; a resident solve's state at that
-                            tick is written to psi_out) */
+                            tick is written to psi_out).  A solve one of whose bounded
+                            device waits gave up fails with GPUE_ERR_TIMEOUT as well,
+                            without a state or an energy */
 } gpue_request;
 
 typedef struct gpue_server_result {
