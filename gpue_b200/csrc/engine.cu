@@ -507,7 +507,7 @@ gpue_status plan_step(gpue_ctx* c, int prec) {
     if (!coop || smem > (size_t)max_smem) return GPUE_OK;
     sc.k = k;
     sc.threads = k->lines * k->p;
-    sc.blocks = (n + k->lines - 1) / k->lines;
+    sc.blocks = n / k->lines;
     sc.smem = smem;
     return GPUE_OK;
 }

@@ -27,8 +27,8 @@
 // What bounds it, and the shapes.  A pass is latency: at 256^2 complex128 it
 // takes about 780 cycles to load, 2200 to transform twice, 1900 in the barrier
 // and 1800 per norm; at 1024^2 complex64 the SMs with most lines issue 85 % of
-// their cycles.  So the lines are dealt out as one CTA per SM (C = n/148
-// rounded up) where a line has at most 32 threads; lines of 64 threads run as
+// their cycles.  So the lines are dealt out as one CTA per SM (C a
+// divisor of n, at least n/148) where a line has at most 32 threads; lines of 64 threads run as
 // several smaller CTAs per SM, whose column barriers then stop 2 to 8 warps
 // instead of all (1024^2 complex64: 42 us per step as 256 CTAs of 4 lines, 48
 // as 147 CTAs of 7).  Time per step on B200, before as line passes and now:
@@ -90,6 +90,9 @@ template <typename T, int N, int RA, int RB, int RC, int P, int C>
 struct StepShape {
     using L = LineFFT<T, N, RA, RB, P, RC>;
     static constexpr int E = L::E;
+    // (else a thread of the last CTA could own a row but no column, and what the
+    // one left in its registers would enter the other's norm)
+    static_assert(N % C == 0, "every CTA holds C whole rows and C whole columns");
     // line stride: the C columns a warp touches at once (16 or 8 lanes at a time)
     // on distinct banks
     static constexpr int W = sizeof(T) == 4 ? 16 : 8;
@@ -263,15 +266,11 @@ __global__ void __launch_bounds__(MAXT, MINB)
     const int tr = tid % P, cr = tid / P;
     const int cc = tid % C, tc = tid / C;
     const int row = rank * C + cr, col = rank * C + cc;
-    // (the last CTA may hold fewer lines: the threads past the field compute on
-    // zeros and neither load nor store)
-    const bool row_ok = row < N, col_ok = col < N;
     // the other axis' factors at the CTA's own row and column
-    const cx<double> lfv = ld2(a.vfac[1], row_ok ? row : 0);
-    const cx<double> lfk = ld2(a.kfac[0], col_ok ? col : 0);
+    const cx<double> lfv = ld2(a.vfac[1], row);
+    const cx<double> lfk = ld2(a.kfac[0], col);
     // the rotation gauge's angles per momentum index along the row and column
-    const double ang[2] = {s.gauge_ang[0] * a.pos[1][row_ok ? row : 0],
-                           s.gauge_ang[1] * a.pos[0][col_ok ? col : 0]};
+    const double ang[2] = {s.gauge_ang[0] * a.pos[1][row], s.gauge_ang[1] * a.pos[0][col]};
     if constexpr (!TAB) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
@@ -312,8 +311,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                 else asm volatile("bar.sync %0, %1;" ::"r"(1 + c), "n"(P) : "memory");
             }
         };
-        const bool line_ok = colpass ? col_ok : row_ok;
-        if ((sp.flags & SP_LOAD) && line_ok) {
+        if (sp.flags & SP_LOAD) {
             const cx<T>* in = static_cast<const cx<T>*>(a.in) + base;
 #pragma unroll
             for (int e = 0; e < E; ++e) {
@@ -354,7 +352,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                         if (a.vtab) {
 #pragma unroll
                             for (int e = 0; e < E; ++e) {
-                                const double V = line_ok ? a.vtab[base + L::index(t, e) * stride] : 0.0;
+                                const double V = a.vtab[base + L::index(t, e) * stride];
                                 const double an = V * (a.step_dt / (2.0 * a.hbar));
                                 const double gd =
                                     a.gpe ? a.nl_coef * ((double)v[e].x * v[e].x +
@@ -394,8 +392,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 #pragma unroll
                             for (int e = 0; e < E; ++e) {
                                 const int i = L::index(t, e);
-                                const double an =
-                                    line_ok ? a.atab[g][base + i * stride] * mom[i] * a.gauge_dt : 0.0;
+                                const double an = a.atab[g][base + i * stride] * mom[i] * a.gauge_dt;
                                 if (gstate == 0)
                                     v[e] = apply_re(v[e], small_decay<T>(an) * a.gscale);
                                 else
@@ -424,7 +421,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                 for (int e = 0; e < E; ++e) v[e].y = -v[e].y;
             }
         }
-        if ((sp.flags & SP_STORE) && line_ok) {
+        if (sp.flags & SP_STORE) {
             cx<T>* out = static_cast<cx<T>*>(a.out) + base;
 #pragma unroll
             for (int e = 0; e < E; ++e) {
