@@ -1214,6 +1214,11 @@ gpue_status step_args(gpue_ctx* c, int prec, int gstate, const std::vector<StepP
     s.target_norm = c->scal + kTargetImag;
     s.target_guard = c->scal + kTargetReal;
     s.err = c->dflags + 3;
+    // (the test hook: "barrier" or "norm" makes that kind of wait run out)
+    const char* hook = std::getenv("GPUE_TEST_STEP_WAIT");
+    s.wait_ns = hook ? 100000000ull : kStepWaitNs;
+    s.more_ctas = hook && !std::strcmp(hook, "barrier") ? 1u << 20 : 0u;
+    s.more_passes = hook && !std::strcmp(hook, "norm") ? 1u << 20 : 0u;
     s.nseq = (int)walk.size();
     std::copy(walk.begin(), walk.end(), s.seq);
     return GPUE_OK;

@@ -44,7 +44,7 @@
 namespace gpue {
 
 constexpr int kStepMaxSeq = 1280;
-constexpr uint64_t kStepWaitNs = 4000000000ull;  // a barrier waits at most 4 s
+constexpr unsigned long long kStepWaitNs = 4000000000ull;  // a wait gives up after 4 s
 
 // One pass of the walk: up to 8 op codes (4 bits each, first in the low bits)
 // and its flags.
@@ -73,6 +73,9 @@ struct StepArgs {
     const double* target_norm;
     const double* target_guard;
     int* err;
+    unsigned long long wait_ns;  // a wait gives up after this long
+    unsigned more_ctas;          // barriers wait for, norms ask for: 0, or (GPUE_TEST_STEP_WAIT,
+    unsigned more_passes;        // tests only) more than ever come, so every such wait runs out
     int nseq;
     StepPass seq[kStepMaxSeq];
 };
@@ -120,7 +123,8 @@ __device__ __forceinline__ uint64_t step_ns() {
 }
 
 // All CTAs of the team arrive and wait; false when the wait ran out.
-__device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, StepShared* sh) {
+__device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, uint64_t limit_ns,
+                                             StepShared* sh) {
     __syncthreads();  // every thread's stores before thread 0's release
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
@@ -132,7 +136,7 @@ __device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, S
             if ((++polls & 1023u) == 0u) {
                 const uint64_t now = step_ns();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > kStepWaitNs) {
+                else if (now - t0 > limit_ns) {
                     sh->abort = 1;
                     break;
                 }
@@ -165,7 +169,7 @@ __device__ __forceinline__ unsigned long long slot_load(const double2* p, double
 // The sum of all CTAs' partials of pass `id`, in a fixed order, by one warp: a
 // lane reads its slots in one batch until all carry the pass's number.
 __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigned long long id,
-                                            StepShared* sh) {
+                                            uint64_t limit_ns, StepShared* sh) {
     constexpr int B = 5;  // 148 CTAs in one batch
     const int lane = threadIdx.x & 31;
     KSum r{0.0, 0.0};
@@ -184,7 +188,7 @@ __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigne
             if ((++polls & 1023u) == 0u) {
                 const uint64_t now = step_ns();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > kStepWaitNs) {
+                else if (now - t0 > limit_ns) {
                     sh->abort = 1;
                     break;
                 }
@@ -440,13 +444,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
         }
         if (flags & SP_SYNC) {
             target += (unsigned)ncta;
-            if (!step_barrier(s.sync, target, sh)) break;
+            if (!step_barrier(s.sync, target + s.more_ctas, s.wait_ns, sh)) break;
         }
         if (flags & (SP_NORM | SP_GUARD)) {
             // (a CTA overwrites its slot at the next norm only, and a barrier
             // that every reader of this one has reached lies between)
             if (tid < 32) {
-                const double sum = slots_sum(s.slots, ncta, (unsigned long long)k + 1, sh);
+                const double sum =
+                    slots_sum(s.slots, ncta, (unsigned long long)k + 1 + s.more_passes, s.wait_ns, sh);
                 if (tid == 0) {
                     if (flags & SP_NORM) sh->scale = sqrt(sh->target_norm / sum);
                     else sh->guard = sqrt(sh->target_guard / sum);
