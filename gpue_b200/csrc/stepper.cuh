@@ -15,9 +15,9 @@
 //   - twiddles (the per-stage table) and the per-axis factors sit in shared
 //     memory, the line factors and the gauge constants of the CTA's own lines
 //     are formed once per launch;
-//   - reductions: every CTA leaves its FP64 partial with the pass's number in
-//     one 16-byte slot, and every CTA reads all slots and sums them in the same
-//     order, so all hold the same factor after one hop and no barrier.
+//   - reductions: every CTA leaves its compensated FP64 partial with the pass's
+//     number in one 16-byte slot, and every CTA reads all slots and sums them in
+//     the same order, so all hold the same factor after one hop and no barrier.
 //
 // Barriers wait on CTAs of the same launch only, which a cooperative launch
 // makes resident together.  Every wait is bounded in time: one that gives up
@@ -66,8 +66,7 @@ struct StepArgs {
     PassArgs a;            // field, tables and constants (per-pass fields unused)
     double gauge_ang[2];   // gauge angle per momentum index and unit position, x and y pass
     unsigned* sync;        // [0] barrier count, [1] CTAs finished; zero between launches
-    double2* slots;        // one per CTA: (norm partial, pass number); numbers zero between
-                           // launches
+    double2* slots;        // one per CTA (slot_store); zero between launches
     double* scal_norm;     // the renormalisation factor, read at the start, written at the end
     double* scal_guard;
     const double* target_norm;
@@ -148,41 +147,48 @@ __device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, u
 }
 
 // A slot is written and read as one 16-byte access, so a reader that sees the
-// pass number sees the partial of that pass.
-__device__ __forceinline__ void slot_store(double2* p, double v, unsigned long long id) {
+// pass number sees the partial of that pass: the sum, and its compensation with
+// the pass number in the low 16 of its 52 fraction bits (the compensation is at
+// most 2^-53 of the sum, so they stand below 2^-89 of it).
+constexpr unsigned long long kSlotPass = 0xffffull;
+static_assert(kStepMaxSeq < (int)kSlotPass, "pass numbers fit a slot");
+__device__ __forceinline__ void slot_store(double2* p, KSum v, unsigned pass) {
+    const unsigned long long c =
+        ((unsigned long long)__double_as_longlong(v.c) & ~kSlotPass) | pass;
     asm volatile(
         "{ .reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q; }" ::"l"(p),
-        "l"(__double_as_longlong(v)), "l"(id)
+        "l"(__double_as_longlong(v.s)), "l"(c)
         : "memory");
 }
-__device__ __forceinline__ unsigned long long slot_load(const double2* p, double& v) {
+__device__ __forceinline__ unsigned slot_load(const double2* p, KSum& v) {
     long long a;
-    unsigned long long id;
+    unsigned long long c;
     asm volatile("{ .reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q; }"
-                 : "=l"(a), "=l"(id)
+                 : "=l"(a), "=l"(c)
                  : "l"(p)
                  : "memory");
-    v = __longlong_as_double(a);
-    return id;
+    v.s = __longlong_as_double(a);
+    v.c = __longlong_as_double((long long)(c & ~kSlotPass));
+    return (unsigned)(c & kSlotPass);
 }
 
-// The sum of all CTAs' partials of pass `id`, in a fixed order, by one warp: a
+// The sum of all CTAs' partials of a pass, in a fixed order, by one warp: a
 // lane reads its slots in one batch until all carry the pass's number.
-__device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigned long long id,
+__device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigned pass,
                                             uint64_t limit_ns, StepShared* sh) {
     constexpr int B = 5;  // 148 CTAs in one batch
     const int lane = threadIdx.x & 31;
     KSum r{0.0, 0.0};
     uint64_t t0 = 0;
     for (int first = lane; first < n; first += 32 * B) {
-        double q[B];
+        KSum q[B];
         unsigned polls = 0;
         for (;;) {
             bool ready = true;
 #pragma unroll
             for (int b = 0; b < B; ++b) {
-                q[b] = 0.0;
-                if (first + 32 * b < n) ready &= slot_load(slots + first + 32 * b, q[b]) == id;
+                q[b] = KSum{0.0, 0.0};
+                if (first + 32 * b < n) ready &= slot_load(slots + first + 32 * b, q[b]) == pass;
             }
             if (ready) break;
             if ((++polls & 1023u) == 0u) {
@@ -195,7 +201,7 @@ __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigne
             }
         }
 #pragma unroll
-        for (int b = 0; b < B; ++b) r.add(q[b]);
+        for (int b = 0; b < B; ++b) r.merge(q[b].s, q[b].c);
     }
     __syncwarp();
 #pragma unroll
@@ -440,7 +446,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         if (k + 1 < s.nseq) sp = s.seq[k + 1];  // its latency under the barrier
         if (flags & (SP_NORM | SP_GUARD)) {
             const KSum b = block_reduce(acc, sh->scratch);
-            if (tid == 0) slot_store(s.slots + rank, b.s + b.c, (unsigned long long)k + 1);
+            if (tid == 0) slot_store(s.slots + rank, b, (unsigned)k + 1);
         }
         if (flags & SP_SYNC) {
             target += (unsigned)ncta;
@@ -451,7 +457,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
             // that every reader of this one has reached lies between)
             if (tid < 32) {
                 const double sum =
-                    slots_sum(s.slots, ncta, (unsigned long long)k + 1 + s.more_passes, s.wait_ns, sh);
+                    slots_sum(s.slots, ncta, (unsigned)k + 1 + s.more_passes, s.wait_ns, sh);
                 if (tid == 0) {
                     if (flags & SP_NORM) sh->scale = sqrt(sh->target_norm / sum);
                     else sh->guard = sqrt(sh->target_guard / sum);
@@ -473,7 +479,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         __threadfence();
         if (atomicAdd(s.sync + 1, 1u) == (unsigned)ncta - 1u) {
             s.sync[0] = 0u;
-            for (int i = 0; i < ncta; ++i) s.slots[i] = make_double2(0.0, 0.0);
+            for (int i = 0; i < ncta; ++i) s.slots[i] = make_double2(0.0, 0.0);  // pass 0: none
             __threadfence();
             s.sync[1] = 0u;
         }
