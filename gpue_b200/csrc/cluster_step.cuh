@@ -14,9 +14,9 @@
 // solve never waits for another.
 //
 // A solve's arithmetic does not depend on CS: the transforms and factors are
-// per line, and a norm is formed as one FP64 sum per line, in a fixed order
-// over the line's threads, then summed over the lines in a fixed order by every
-// CTA (blockDim is fixed per length).  So the same solve ends bit for bit the
+// per line, and a norm is formed as one compensated FP64 sum per line, in a fixed
+// order over the line's threads, then summed over the lines in a fixed order by
+// every CTA (blockDim is fixed per length).  So the same solve ends bit for bit the
 // same whatever cluster size a batch gives it.
 //
 // What bounds it: about 313 instructions per point and step, issued at 0.39 to
@@ -82,7 +82,7 @@ struct ClusterShape {
     static constexpr size_t FACB = (size_t)N * 2 * sizeof(T);
     static size_t smem(int cs) {
         const int R = (N + cs - 1) / cs;
-        return sizeof(ClusterShared) + sizeof(ClusterArgs) + TW + 2 * FACB + (size_t)N * 8 +
+        return sizeof(ClusterShared) + sizeof(ClusterArgs) + TW + 2 * FACB + (size_t)N * 16 +
                (size_t)THREADS * 8 + (size_t)R * XS * sizeof(cx<T>) +
                (size_t)LPR * LSC * sizeof(cx<T>) + 64;
     }
@@ -97,9 +97,12 @@ __device__ __forceinline__ void dsmem_store(unsigned addr, cx<T> v) {
         asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y)
                      : "memory");
 }
-__device__ __forceinline__ double dsmem_load_f64(unsigned addr) {
-    double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+__device__ __forceinline__ double2 dsmem_load_f64x2(unsigned addr) {
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];"
+                 : "=d"(v.x), "=d"(v.y)
+                 : "r"(addr)
+                 : "memory");
     return v;
 }
 __device__ __forceinline__ unsigned cluster_ctas() {
@@ -130,8 +133,8 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
     p += S_::FACB;
     Fac* ky_s = reinterpret_cast<Fac*>(p);
     p += S_::FACB;
-    double* line_s = reinterpret_cast<double*>(p);  // [N]: norm of each of this CTA's lines
-    p += (size_t)N * 8;
+    double2* line_s = reinterpret_cast<double2*>(p);  // [N]: (sum, compensation) of this CTA's lines
+    p += (size_t)N * 16;
     double* part_s = reinterpret_cast<double*>(p);  // [THREADS]
     p += (size_t)S_::THREADS * 8;
     cx<T>* X = reinterpret_cast<cx<T>*>(p);  // [R][XS]
@@ -282,18 +285,21 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
                 }
             }
             if (norm) {
-                // one FP64 sum per line, in the order of its threads
+                // one compensated sum per line, in the order of its threads
                 __syncthreads();  // the previous round's sums are read
-                part_s[l0 * P + t] = acc.s + acc.c;
+                part_s[l0 * P + t] = acc.s + acc.c;  // (one term: exact)
                 __syncthreads();
-                double q = part_s[tid];
+                KSum q{part_s[tid], 0.0};
                 if constexpr (P > 32) {
-                    if (tr < 32) q += part_s[tid + 32];
+                    if (tr < 32) q.add(part_s[tid + 32]);
                 }
 #pragma unroll
-                for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1)
-                    q += __shfl_down_sync(0xffffffffu, q, o, P < 32 ? P : 32);
-                if (tr == 0 && base + lr < mine) line_s[base + lr] = q;
+                for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) {
+                    const double os = __shfl_down_sync(0xffffffffu, q.s, o, P < 32 ? P : 32);
+                    const double oc = __shfl_down_sync(0xffffffffu, q.c, o, P < 32 ? P : 32);
+                    q.merge(os, oc);
+                }
+                if (tr == 0 && base + lr < mine) line_s[base + lr] = make_double2(q.s, q.c);
             }
         }
         const unsigned flags = sp.flags;
@@ -307,7 +313,8 @@ __device__ __forceinline__ void cluster_steps(const Args& s, const StepPass* __r
             KSum r{0.0, 0.0};
             for (int i = tid; i < N; i += S_::THREADS) {
                 const unsigned q = __umulhi((unsigned)i, Rmul);
-                r.add(dsmem_load_f64(dsmem_map(smem_addr(line_s) + (i - q * R) * 8, q)));
+                const double2 ls = dsmem_load_f64x2(dsmem_map(smem_addr(line_s) + (i - q * R) * 16, q));
+                r.merge(ls.x, ls.y);
             }
             r = block_reduce(r, sh->scratch);
             if (tid == 0) {
