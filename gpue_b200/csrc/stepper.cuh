@@ -108,7 +108,7 @@ struct StepShape {
     static constexpr size_t TW = (size_t)L::kStageTableLen * 16;
     static constexpr size_t FACB = FAC ? (size_t)N * 2 * sizeof(T) : 0;  // one factor table
     static constexpr size_t fixed_bytes() { return sizeof(StepShared) + TW + 2 * FACB; }
-    // per thread: W^t of the two gauge passes; per line: A, B, W^-n of both
+    // per thread: W^t of the two gauge passes; per line: A, B, W^(-n/2) of both
     static size_t smem(int) {
         return fixed_bytes() + (size_t)NBUF * C * LS * sizeof(cx<T>) + (size_t)C * P * 32 +
                (size_t)C * 96;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                 cx<double>* gl = gl_s + (g * C + c) * 3;
                 gl[0] = gc.wa;
                 gl[1] = gc.wb;
-                gl[2] = gc.wn;
+                gl[2] = gc.wh;
             }
         }
     }
