@@ -310,14 +310,15 @@ struct LineFFT {
     // shared-memory access is served 16 lanes (complex64) or 8 (complex128) at a
     // time.  Rows (LS): lanes are a line's threads, so only complex64 lines of 8
     // threads share a group, 8 elements apart.  Strided passes (LSC): lanes are C
-    // adjacent lines (C = 128/P in the default launch shape) by 16/C or 8/C
-    // threads, so the lines lie that many elements apart.  With one offset of 4 for
+    // adjacent lines (in the default launch shape C = 128/P, but 4 complex64 lines
+    // of 64 threads) by 16/C or 8/C threads, so the lines lie that many elements
+    // apart.  With one offset of 4 for
     // all, complex128 columns of 8-thread lines met 4 to a bank: per step on B200
     // 96^3 complex128 56 -> 47 us, rotating 82 -> 64, 160^3 complex64 113 -> 103.
     static constexpr int kPad16 = ((phys(N - 1) + 1 + 15) / 16) * 16;
     static constexpr int LS = kPad16 + (sizeof(T) == 4 && P == 8 ? 8 : 4);
     static constexpr int LSC =
-        kPad16 + (sizeof(T) == 4 ? (P >= 16 ? P / 8 : 1) : (P >= 32 ? P / 16 : 1));
+        kPad16 + (sizeof(T) == 4 ? (P >= 32 ? 4 : P >= 16 ? 2 : 1) : (P >= 32 ? P / 16 : 1));
     static constexpr int LSMAX = LS > LSC ? LS : LSC;
 
     __host__ __device__ static constexpr int radix(int s) {

@@ -619,8 +619,11 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
     if constexpr (STRIDED) {
         c = threadIdx.x % C;
         // (blockDim.x = C P: the mask changes nothing, but the known range lets
-        // the compiler fold the exchanges' padded offsets into constants)
-        t = (threadIdx.x / C) & (P - 1);
+        // the compiler fold the exchanges' padded offsets into constants; with 64
+        // threads a line complex128 spills more for it, 4 batched 1024^2 372 us per
+        // step without and 380 with)
+        t = threadIdx.x / C;
+        if (sizeof(T) == 4 || P < 64) t &= P - 1;
     } else {
         t = threadIdx.x % P;
         c = threadIdx.x / P;
@@ -797,7 +800,13 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     const int src = a.gauge_src;
                     const int sidx = (src == 0) ? xi : (src == 1) ? yi : zi;
                     const double ang1 = a.gauge_coef * a.pos[src][sidx] * a.gauge_dt * a.dmom;
-                    op_gauge<T, L>(v, gauge_consts<L>(t, ang1, a.gstate, a.gscale), a.gstate);
+                    // (one branch per time kind, so that only its own constants are
+                    // held: with both the 640 complex64 column pass spilled 524 bytes
+                    // instead of 364, 8 batched 640^2 151 us per step instead of 144)
+                    if (a.gstate == 0)
+                        op_gauge<T, L>(v, gauge_consts<L>(t, ang1, 0, a.gscale), 0);
+                    else
+                        op_gauge<T, L>(v, gauge_consts<L>(t, ang1, 1, a.gscale), 1);
                     break;
                 }
                 case OP_NORM:
