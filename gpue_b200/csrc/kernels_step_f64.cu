@@ -2,11 +2,12 @@
 //
 // (length, radix plan, threads per line, lines per CTA, CTAs per SM).  One CTA per
 // SM where the lines have at most 32 threads; the plans are the line passes'
-// defaults except where one with fewer exchanges or CTAs was faster in a resident
-// walk: 128 (8 2 8; complex128 rotating 13.4 -> 12.4 us per step), 320 (4 20 4
-// instead of 4 5 4 4; 25.6 -> 23.3) and 768 (8 12 8 with 32 threads instead of 4
-// 12 4 4 with 64; 51.6 -> 47.6, complex64 in imaginary time 23.2 -> 20.7).  16 16
-// at 256 and 8 8 8 with 32 threads at 512 were slower (9.4 -> 10.7, 15.4 -> 16.3).
+// defaults, so a step is as far from the exact one as they are.  Two others were
+// faster and are not used: 8 2 8 at 128 (complex128 rotating 12.4 us per step
+// instead of 13.4) is 1.3 to 1.6 times as far from the step in 80-bit arithmetic
+// (complex64 1.08 times from complex128), 8 12 8 at 768 (47.6 instead of 51.6) up
+// to 1.05 times.  16 16 at 256 and 8 8 8 with 32 threads at 512 were slower (9.4
+// -> 10.7, 15.4 -> 16.3).
 #include "stepper.cuh"
 
 namespace gpue {
@@ -16,7 +17,7 @@ static const StepKernel kTable[] = {
     GPUE_STEP(double, 32, 4, 2, 0, 8, 4, 1),
     GPUE_STEP(double, 64, 4, 4, 0, 16, 2, 1),
     GPUE_STEP(double, 96, 4, 6, 0, 8, 4, 1),
-    GPUE_STEP(double, 128, 8, 2, 0, 16, 2, 1),
+    GPUE_STEP(double, 128, 4, 8, 0, 16, 2, 1),
     GPUE_STEP(double, 160, 4, 10, 0, 8, 4, 1),
     GPUE_STEP(double, 192, 4, 12, 0, 16, 2, 1),
     GPUE_STEP(double, 256, 8, 4, 0, 32, 2, 1),
@@ -24,7 +25,7 @@ static const StepKernel kTable[] = {
     GPUE_STEP(double, 384, 4, 6, 4, 32, 3, 1),
     GPUE_STEP(double, 512, 8, 8, 0, 64, 2, 2),
     GPUE_STEP(double, 640, 4, 10, 4, 32, 5, 1),
-    GPUE_STEP(double, 768, 8, 12, 0, 32, 6, 1),
+    GPUE_STEP(double, 768, 4, 12, 4, 64, 2, 3),
     GPUE_STEP(double, 1024, 16, 4, 0, 64, 4, 2),
 };
 
