@@ -73,10 +73,10 @@ __device__ __forceinline__ double gauge_energy(const EnergyArgs& a, const cx<T>*
 // Rows of nx points dealt to `ncta` CTAs of 256 threads: tpr threads (a power of
 // two) share a row and a thread takes B rows at a time, whose loads are requested
 // together.  The y and z indices advance by addition.  f(psi value, x, y, z, flat
-// index) for every point, done() after each batch of rows.
-template <int B, typename T, class F, class D>
+// index) for every point.
+template <int B, typename T, class F>
 __device__ __forceinline__ void for_rows(const cx<T>* psi, int nx, int ny, int rows, int cta,
-                                         int ncta, F f, D done) {
+                                         int ncta, F f) {
     int tpr = 32;
     while (tpr < nx && tpr < 256) tpr *= 2;
     const int per = 256 / tpr, lane = (int)threadIdx.x & (tpr - 1);
@@ -108,7 +108,6 @@ __device__ __forceinline__ void for_rows(const cx<T>* psi, int nx, int ny, int r
             for (int k = 0; k < B; ++k)
                 if (k < full) f(p[k], x, yk[k], zk[k], g + k * stride);
         }
-        done();
     }
 }
 
@@ -124,7 +123,6 @@ __device__ __forceinline__ KSum energy_real_points(const EnergyArgs& a, int cta,
     const double hg = a.gpe ? 0.5 * a.gN : 0.0;
     const long nxy = (long)a.nx * a.ny;
     KSum acc{0.0, 0.0};
-    double part = 0.0;  // a batch's terms in plain FP64, then into the compensated sum
     for_rows<PLAIN ? 4 : 1>(
         psi, a.nx, a.ny, (int)(a.N / a.nx), cta, ncta,
         [&](cx<T> pv, int xi, int yi, int zi, long g) {
@@ -132,17 +130,14 @@ __device__ __forceinline__ KSum energy_real_points(const EnergyArgs& a, int cta,
             const double r = px * px + py * py;
             if constexpr (PLAIN) {
                 const double V = a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-                part += r * (V + hg * r);
+                acc.add(r * (V + hg * r));
             } else {
                 const double V =
                     a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-                part += r * (V + hg * r);
-                if (a.lterm) part += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+                double e = r * (V + hg * r);
+                if (a.lterm) e += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+                acc.add(e);
             }
-        },
-        [&] {
-            acc.add(part);
-            part = 0.0;
         });
     return acc;
 }
@@ -202,7 +197,6 @@ __global__ void __launch_bounds__(256, 2) k_observables(const ObsArgs o) {
     KSum acc[kObsN];
 #pragma unroll
     for (int q = 0; q < kObsN; ++q) acc[q] = KSum{0.0, 0.0};
-    double part[kObsN] = {};  // a batch's terms in plain FP64
     for_rows<1>(
         psi, a.nx, a.ny, (int)(a.N / a.nx), blockIdx.x, gridDim.x,
         [&](cx<T> pv, int xi, int yi, int zi, long g) {
@@ -210,33 +204,26 @@ __global__ void __launch_bounds__(256, 2) k_observables(const ObsArgs o) {
             const double r = px * px + py * py;
             const double V =
                 a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-            part[kObsNorm] += r;
-            part[kObsPot] += r * V;
-            if (a.gpe) part[kObsInt] += 0.5 * a.gN * r * r;
-            if (a.lterm) part[kObsRot] += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+            acc[kObsNorm].add(r);
+            acc[kObsPot].add(r * V);
+            if (a.gpe) acc[kObsInt].add(0.5 * a.gN * r * r);
+            if (a.lterm) acc[kObsRot].add(gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py));
             const double X = a.pos[0][xi];
             const double Y = a.dim > 1 ? a.pos[1][yi] : 0.0;
             const double Z = a.dim > 2 ? a.pos[2][zi] : 0.0;
             const double wr = r * trapz_w(xi, a.nx) * trapz_w(yi, a.ny) * trapz_w(zi, a.nz);
-            part[kObsX] += wr * X;
-            part[kObsY] += wr * Y;
-            part[kObsZ] += wr * Z;
-            part[kObsR2] += wr * (X * X + Y * Y);
-            part[kObsQ] += wr * (X * X - Y * Y);
+            acc[kObsX].add(wr * X);
+            acc[kObsY].add(wr * Y);
+            acc[kObsZ].add(wr * Z);
+            acc[kObsR2].add(wr * (X * X + Y * Y));
+            acc[kObsQ].add(wr * (X * X - Y * Y));
             if (a.dim > 1) {
                 // -i hbar (x d+y - y d+x) psi, then Re[conj(p) * that]
                 double dxr, dxi, dyr, dyi;
                 dfwd(psi, a.N, g, 1, s, px, py, a.dx, dxr, dxi);
                 dfwd(psi, a.N, g, a.nx, s, px, py, a.dy, dyr, dyi);
                 const double Dr = X * dyr - Y * dxr, Di = X * dyi - Y * dxi;
-                part[kObsLz] += a.hbar * (px * Di - py * Dr);
-            }
-        },
-        [&] {
-#pragma unroll
-            for (int q = 0; q < kObsN; ++q) {
-                acc[q].add(part[q]);
-                part[q] = 0.0;
+                acc[kObsLz].add(a.hbar * (px * Di - py * Dr));
             }
         });
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -381,10 +368,8 @@ __global__ void __launch_bounds__(256) k_norm(void* psi_, long N, const double* 
                 if (g + k * step < N) psi[g + k * step] = v[k];
             }
         }
-        double part = 0.0;  // four terms in plain FP64, then into the compensated sum
 #pragma unroll
-        for (int k = 0; k < 4; ++k) part += (double)v[k].x * v[k].x + (double)v[k].y * v[k].y;
-        acc.add(part);
+        for (int k = 0; k < 4; ++k) acc.add((double)v[k].x * v[k].x + (double)v[k].y * v[k].y);
     }
     grid_reduce_finish(acc, scratch, red, gridDim.x, blockIdx.x);
 }
