@@ -111,39 +111,51 @@ __device__ __forceinline__ void for_rows(const cx<T>* psi, int nx, int ny, int r
     }
 }
 
-// PLAIN: separable V and no gauge term, the form of most checks, in few enough
-// registers for four CTAs per SM and four rows in flight per thread: 256^3 takes
-// 55 us in complex64 and 61 in complex128.  With the gauge term's six divisions
-// per point inlined beside it the kernel held one CTA per SM (224 us); one point
-// at a time with 64-bit index divisions it took 112 us.
+// The terms of CTA `cta` of `ncta`.  PLAIN: separable V and no gauge term, the form
+// of most checks, in few enough registers for four CTAs per SM and four rows in
+// flight per thread: 256^3 takes 66 us in complex64 and 68 in complex128, 112 a
+// point at a time with 64-bit index divisions.  The general form keeps those: by
+// rows its gauge term's neighbours and divisions take more registers (an energy
+// call on a rotating 256^3 complex64 state 522 us a point at a time, 604 by rows).
 template <typename T, bool PLAIN>
 __device__ __forceinline__ KSum energy_real_points(const EnergyArgs& a, int cta, int ncta) {
     const cx<T>* psi = reinterpret_cast<const cx<T>*>(a.psi);
     const double s = a.scale ? *a.scale : 1.0;
-    const double hg = a.gpe ? 0.5 * a.gN : 0.0;
-    const long nxy = (long)a.nx * a.ny;
     KSum acc{0.0, 0.0};
-    for_rows<PLAIN ? 4 : 1>(
-        psi, a.nx, a.ny, (int)(a.N / a.nx), cta, ncta,
-        [&](cx<T> pv, int xi, int yi, int zi, long g) {
+    if constexpr (PLAIN) {
+        const double hg = a.gpe ? 0.5 * a.gN : 0.0;
+        for_rows<4>(psi, a.nx, a.ny, (int)(a.N / a.nx), cta, ncta,
+                    [&](cx<T> pv, int xi, int yi, int zi, long) {
+                        const double px = s * (double)pv.x, py = s * (double)pv.y;
+                        const double r = px * px + py * py;
+                        const double V = a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
+                        acc.add(r * (V + hg * r));
+                    });
+    } else {
+        const long nxy = (long)a.nx * a.ny, step = (long)ncta * blockDim.x;
+        for (long g = (long)cta * blockDim.x + threadIdx.x; g < a.N; g += step) {
+            const int xi = (int)(g % a.nx);
+            const int yi = (int)((g / a.nx) % a.ny);
+            const int zi = (int)(g / nxy);
+            const cx<T> pv = psi[g];
             const double px = s * (double)pv.x, py = s * (double)pv.y;
             const double r = px * px + py * py;
-            if constexpr (PLAIN) {
-                const double V = a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-                acc.add(r * (V + hg * r));
-            } else {
-                const double V =
-                    a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
-                double e = r * (V + hg * r);
-                if (a.lterm) e += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
-                acc.add(e);
-            }
-        });
+            const double V =
+                a.vtab ? a.vtab[g] : a.vreal[0][xi] + a.vreal[1][yi] + a.vreal[2][zi];
+            double e = a.gpe ? r * (V + 0.5 * a.gN * r) : r * V;
+            if (a.lterm) e += gauge_energy<T>(a, psi, g, xi, yi, nxy, s, px, py);
+            acc.add(e);
+        }
+    }
     return acc;
 }
 
+// (the general form is left to the compiler's own choice of registers, 64)
+constexpr int energy_min_blocks(bool plain) { return plain ? 4 : 0; }
+
 template <typename T, bool PLAIN>
-__global__ void __launch_bounds__(256, PLAIN ? 4 : 2) k_energy_real(const EnergyArgs a) {
+__global__ void __launch_bounds__(256, energy_min_blocks(PLAIN))
+    k_energy_real(const EnergyArgs a) {
     __shared__ double scratch[16];
     KSum acc = energy_real_points<T, PLAIN>(a, blockIdx.x, gridDim.x);
     grid_reduce_finish(acc, scratch, a.red, gridDim.x, blockIdx.x);
@@ -151,17 +163,15 @@ __global__ void __launch_bounds__(256, PLAIN ? 4 : 2) k_energy_real(const Energy
 
 // Independent solves at once: `per` CTAs per solve, each solve reducing over
 // its own CTAs; converged solves (*active == 0) are skipped.
-template <typename T>
-__global__ void __launch_bounds__(256, 3) k_energy_real_batch(const EnergyArgs* __restrict__ args,
-                                                          const int* const* __restrict__ active,
-                                                          int per) {
+template <typename T, bool PLAIN>
+__global__ void __launch_bounds__(256, energy_min_blocks(PLAIN))
+    k_energy_real_batch(const EnergyArgs* __restrict__ args,
+                        const int* const* __restrict__ active, int per) {
     __shared__ double scratch[16];
     const int s = blockIdx.x / per, b = blockIdx.x % per;
     if (active[s] && *active[s] == 0) return;
     const EnergyArgs& a = args[s];
-    const bool plain = !a.lterm && !a.vtab;
-    KSum acc = plain ? energy_real_points<T, true>(a, b, per)
-                     : energy_real_points<T, false>(a, b, per);
+    KSum acc = energy_real_points<T, PLAIN>(a, b, per);
     grid_reduce_finish(acc, scratch, a.red, per, b);
 }
 

@@ -522,11 +522,15 @@ gpue_status plan_segment(const BatchRun& r, int s0, int s1, bool check, ArgSink&
             const unsigned grid = (unsigned)(n * per);
             const int iper = (int)per;
             const bool f32 = g.prec == GPUE_PREC_FP32;
+            bool plain = true;
+            for (const EnergyArgs& e : ea) plain &= !e.lterm && !e.vtab;
             out_ops.push_back([=](cudaStream_t s) {
                 const EnergyArgs* e = static_cast<const EnergyArgs*>(dea);
                 const int* const* a = static_cast<const int* const*>(dact);
-                if (f32) k_energy_real_batch<float><<<grid, 256, 0, s>>>(e, a, iper);
-                else k_energy_real_batch<double><<<grid, 256, 0, s>>>(e, a, iper);
+                if (f32 && plain) k_energy_real_batch<float, true><<<grid, 256, 0, s>>>(e, a, iper);
+                else if (f32) k_energy_real_batch<float, false><<<grid, 256, 0, s>>>(e, a, iper);
+                else if (plain) k_energy_real_batch<double, true><<<grid, 256, 0, s>>>(e, a, iper);
+                else k_energy_real_batch<double, false><<<grid, 256, 0, s>>>(e, a, iper);
             });
             sp.launches++;
         }

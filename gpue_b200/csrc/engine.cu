@@ -920,9 +920,11 @@ gpue_status launch_energy(gpue_ctx* c, int prec, int gstate, bool scale_pending,
         if (prec == GPUE_PREC_FP32) k_observables<float><<<blocks, 256, 0, c->stream>>>(oa);
         else k_observables<double><<<blocks, 256, 0, c->stream>>>(oa);
     } else {
-        const int blocks = (int)std::max(1L, std::min<long>(c->sms * 4, c->N / 1024));
-        const bool f32 = prec == GPUE_PREC_FP32;
-        if (!e.lterm && !e.vtab) {
+        const bool f32 = prec == GPUE_PREC_FP32, plain = !e.lterm && !e.vtab;
+        // (four points a thread and round, or one)
+        const int blocks =
+            (int)std::max(1L, std::min<long>(c->sms * 4, c->N / (plain ? 1024 : 256)));
+        if (plain) {
             if (f32) k_energy_real<float, true><<<blocks, 256, 0, c->stream>>>(e);
             else k_energy_real<double, true><<<blocks, 256, 0, c->stream>>>(e);
         } else {
