@@ -113,12 +113,15 @@ bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
 
 // Cluster sizes of a run's 2D solves (0: not on the cluster stepper).  A solve
 // starts at the smallest cluster that holds its field; while the device has
-// room, the one with most points per CTA doubles, so a mix finishes together
-// and few solves still use the device.  A cluster must lie in one GPC, so the
+// room, those with most points per CTA double, so a mix finishes together and
+// few solves still use the device.  A cluster must lie in one GPC, so the
 // device holds fewer large ones than its SMs suggest (7 of 16 CTAs, not 9):
-// each counts as the share of the device that the occupancy query says.  16
-// solves of 256^2 complex64 as clusters of 8 take two waves, 52 us a step; as
-// clusters of 4, one.  Results do not depend on the choice.
+// each counts as the share of the device that the occupancy query says.  Equal
+// solves double together or not at all: the slowest decide when the launch ends,
+// and two sizes of cluster do not fill the GPCs as their shares suggest (12 of
+// 96^2 complex64 in real time, some as 16 CTAs and some as 8, took two waves, 17.7
+// us a step; as 8 each 9.4, as line passes 16.1).  Results do not depend on the
+// choice.
 std::vector<int> cluster_sizes(const BatchRun& r) {
     const size_t n = r.ctx.size();
     std::vector<int> cs(n, 0);
@@ -155,14 +158,20 @@ std::vector<int> cluster_sizes(const BatchRun& r) {
             }
         }
         if (best < 0) break;
-        const int s = 2 * cs[best];
-        if (s > r.ctx[best]->cluster[r.ctx[best]->prec].cs ||
-            total + share(best, s) - share(best, cs[best]) > 1.0) {
-            full[best] = 1;
-            continue;
+        const int from = cs[best], to = 2 * from;
+        const ClusterKernel* k = r.ctx[best]->cluster[r.ctx[best]->prec].k;
+        std::vector<size_t> equal;
+        for (size_t i = 0; i < n; ++i)
+            if (cs[i] == from && r.ctx[i]->cluster[r.ctx[i]->prec].k == k) equal.push_back(i);
+        const double more = to <= r.ctx[best]->cluster[r.ctx[best]->prec].cs
+                                ? (double)equal.size() * (share(best, to) - share(best, from))
+                                : 2.0;
+        const bool fits = total + more <= 1.0;
+        for (size_t i : equal) {
+            if (fits) cs[i] = to;
+            else full[i] = 1;
         }
-        total += share(best, s) - share(best, cs[best]);
-        cs[best] = s;
+        if (fits) total += more;
     }
     return cs;
 }
