@@ -88,27 +88,35 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
            c->xy[prec].k && c->zpass[prec].k && plane_ok(c, prec);
 }
 
-// 2D solves that run on the grid-wide stepper, one after another.  Complex64 up
-// to 512^2: those too large for a cluster to step quickly alone, 512^2 and 384^2
-// with the gauge (one of 512^2 per step as line passes, as a cluster of 16 and as
-// a grid: 30, 55 and 12 us; rotating 48, 102 and 18; 24 of them 342, 220 and 287,
-// so many alike would be faster on clusters).  From 768 on, line passes in
-// groups and the grid: 8 of 768^2 complex64 218 and 165 us, complex128 306 and
-// 206, 8 of 1024^2 complex64 270 and 197, one 41 and 25, 4 of 1024^2 complex128
-// 232 and 141.  In between the groups are faster as soon as several share them,
-// 8 of 384^2 complex128 70 and 112, 8 of 640^2 198 and 208, 24 of 640^2 complex64
-// 426 and 468, though one alone is not (384^2 complex128 56 and 14).  The choice
-// is the solve's own, never the mix's, so a result does not depend on its company.
+// 2D solves that run on the grid-wide stepper.  Complex64 of 384^2 and 512^2, too
+// large for a cluster to step quickly alone; as many grids as the device holds
+// at once, up to 4, run side by side on lanes of their own (grid_lanes).  Per step
+// as line passes and as grids: one of 512^2 30 and 12 us, 40 of them 368 and 297
+// (one lane: 482), rotating 632 and 469; one of 384^2 42 and 11 (37 as a cluster
+// of 16), 40 of them 329 and 165 (one lane 439, clusters 222), rotating 549 and
+// 268 (729, 409).  From 768 on a grid fills the device, one after another: 8 of
+// 768^2 complex64 208 and 179, complex128 320 and 229, 8 of 1024^2 complex64 270
+// and 197, 4 of 1024^2 complex128 232 and 141.  In between the line passes are
+// faster as soon as several solves share them, 8 of 384^2 complex128 70 and 112
+// us, 8 of 640^2 198 and 208, 24 of 640^2 complex64 393 and 468, though one alone
+// is not (384^2 complex128 56 and 14); 320^2 complex64 on clusters took 29 us
+// alone and 144 as 40, rotating 53 and 267, as line passes 32, 131, 47 and 208.
+// The choice is the solve's own, never the mix's, so a result does not depend on
+// its company.
 bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
     const char* env = std::getenv("GPUE_BATCH_MEGA");
     if (env && env[0] == '0') return false;
     if (c->dim != 2 || !c->step[prec].k || c->ext || c->time_dep || c->line_plan) return false;
-    if (c->ax[0].n < 768) {
-        if (prec != GPUE_PREC_FP32 || c->ax[0].n > 512) return false;
-        const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
-        if (c->N * (gauge ? 2 : 1) < (1L << 18)) return false;
-    }
+    if (c->ax[0].n < 768 && (prec != GPUE_PREC_FP32 || (c->ax[0].n != 384 && c->ax[0].n != 512)))
+        return false;
     return step_ready(c, prec, gstate);
+}
+
+// Lanes of a solve's grid group: the grids of its kind that the device holds at
+// once, at most 4 (40 of 384^2 complex64 439 us per step on one lane, 264 on two,
+// 203 on three, 165 on four; 512^2, two of which fit, 482, 297, 324 and 309).
+int grid_lanes(const gpue_ctx* c, int gstate) {
+    return std::min(4, c->step[c->prec].ready[c->ext ? 1 : 0][gstate ? 1 : 0]);
 }
 
 // Cluster sizes of a run's 2D solves (0: not on the cluster stepper).  A solve
@@ -180,14 +188,16 @@ void group_solves(BatchRun& r, int probe) {
     r.groups.clear();
     std::map<std::string, int> by_sig;
     const std::vector<int> cs = cluster_sizes(r);
+    std::map<std::pair<int, int>, int> grids;  // solves on the grid so far, by length and precision
     for (size_t i = 0; i < r.ctx.size(); ++i) {
         gpue_ctx* c = r.ctx[i];
         const int off = r.offset[i];
         const bool tile = tile_eligible(c, c->prec);
         const bool grid = !cs[i] && grid_eligible(c, c->prec, r.gstate);
+        const int lane = grid ? grids[{c->ax[0].n, c->prec}]++ % grid_lanes(c, r.gstate) : 0;
         const std::string sig =
             std::to_string((int)r.guard[i]) + "/" + (tile ? "tile/" : "") +
-            (cs[i] ? "cluster" + std::to_string(cs[i]) + "/" : "") + (grid ? "grid/" : "") +
+            (cs[i] ? "cluster" + std::to_string(cs[i]) + "/" : "") + (grid ? "grid" + std::to_string(lane) + "/" : "") +
             pass_signature(c, c->prec,
                            solve_passes(c, off, off + probe, r.gstate, r.guard[i], r.scale_step0,
                                         tile));
@@ -385,7 +395,7 @@ static gpue_status plan_cluster_launch(const BatchRun& r, const BGroup& g, int s
 }
 
 // The steps [s0, s1) of a grid group: one cooperative launch per solve (per
-// kStepChunk steps) on the group's lane.
+// kStepChunk steps), one after another on the group's lane.
 static gpue_status plan_grid_launches(const BatchRun& r, const BGroup& g, int s0, int s1,
                                       std::vector<LaunchOp>& ops, long& launches,
                                       std::string& err) {

@@ -35,7 +35,7 @@ struct BGroup {
     bool mega = false;         // its solves run on the persistent multi-size kernel
     int cluster = 0;           // > 0: each solve runs on a cluster of that many CTAs
     bool grid = false;         // each solve runs on the grid-wide 2D stepper, one after another
-    bool tile = false;         // 3D complex64: the three tile-stream passes per step, per solve
+    bool tile = false;         // 3D: the tile-stream passes of each solve, one launch per pass
     std::vector<int> members;  // indices into BatchRun::ctx
 };
 

@@ -528,7 +528,7 @@ bool step_ready(gpue_ctx* c, int prec, int gstate) {
                 cudaSuccess &&
             (long)per_sm * c->sms >= sc.blocks;
         if (!fits) cudaGetLastError();  // not an error of the call that asks
-        r = fits ? 1 : -1;
+        r = fits ? (int)((long)per_sm * c->sms / sc.blocks) : -1;
     }
     return r > 0;
 }

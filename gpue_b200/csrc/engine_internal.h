@@ -120,7 +120,7 @@ struct StepCfg {
     const StepKernel* k = nullptr;
     int threads = 0, blocks = 0;
     size_t smem = 0;
-    int ready[2][2] = {};  // [tables][real time]: 1 the grid is resident at once, -1 it is not
+    int ready[2][2] = {};  // [tables][real time]: grids the device holds at once, -1 none
 };
 
 // The cluster-resident stepper of a 2D context (cluster_step.cuh)

@@ -7,7 +7,8 @@
 // instead of 13.4) is 1.3 to 1.6 times as far from the step in 80-bit arithmetic
 // (complex64 1.08 times from complex128), 8 12 8 at 768 (47.6 instead of 51.6) up
 // to 1.05 times.  16 16 at 256 and 8 8 8 with 32 threads at 512 were slower (9.4
-// -> 10.7, 15.4 -> 16.3).
+// -> 10.7, 15.4 -> 16.3).  384 and 512 leave registers for a second CTA, so
+// batched solves run side by side (batch.cu).
 #include "stepper.cuh"
 
 namespace gpue {
@@ -22,8 +23,8 @@ static const StepKernel kTable[] = {
     GPUE_STEP(float, 192, 4, 12, 0, 16, 2, 1),
     GPUE_STEP(float, 256, 8, 4, 0, 32, 4, 1),
     GPUE_STEP(float, 320, 4, 20, 0, 16, 4, 1),
-    GPUE_STEP(float, 384, 4, 6, 4, 32, 4, 1),
-    GPUE_STEP(float, 512, 8, 8, 0, 64, 4, 1),
+    GPUE_STEP(float, 384, 4, 6, 4, 32, 4, 2),
+    GPUE_STEP(float, 512, 8, 8, 0, 64, 4, 2),
     GPUE_STEP(float, 640, 4, 10, 4, 32, 5, 1),
     GPUE_STEP(float, 768, 4, 12, 4, 64, 2, 3),
     GPUE_STEP(float, 1024, 16, 4, 0, 64, 4, 2),
