@@ -59,10 +59,10 @@
 // Per step of 256^3 complex128, five line passes and these three: 809 -> 426 us;
 // 128^3 125 -> 87; with the gauge 256^3 1170 -> 780, complex64 704 -> 506.
 //
-// The norm in complex128: every warp leaves its FP64 sum of a tile with the
-// producer, which adds the warps' in order into the tile's partial; the last CTA
-// to finish sums all tiles' partials in tile order, so the result does not
-// depend on which CTA took which tile and runs repeat bit for bit.  Complex64
+// The norm in complex128: every warp leaves its compensated FP64 sum of a tile
+// with the producer, which adds the warps' in order into the tile's partial; the
+// last CTA to finish sums all tiles' partials in tile order, so the result does
+// not depend on which CTA took which tile and runs repeat bit for bit.  Complex64
 // keeps one compensated sum per thread (the per-tile sums cost 1.2 % there).
 #pragma once
 
@@ -99,7 +99,7 @@ struct TSShape {
     // partials of the two tiles, + 1024 bytes to align the base (the 128-byte
     // swizzle repeats every 1024 bytes of the destination address)
     static constexpr size_t OFF_NRM = OFF_BAR + 96;
-    static constexpr size_t SMEM = OFF_NRM + 2 * CW * 8 + 1024;
+    static constexpr size_t SMEM = OFF_NRM + (sizeof(T) == 8 ? 2 * CW * 16 : 0) + 1024;
     // resident CTAs: complex64 measured no faster with more than two (160^3 in
     // real time 113 us per step with two, 118 with three); complex128 tiles of
     // the short lengths hold few warps, so as many as fit
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS,
     // the first and second tile kind of an XY pass
     constexpr bool YX = KIND == TS_YX_INV_GX;
     constexpr int K1 = YX ? TILE_Y : TILE_X, K2 = YX ? TILE_X : TILE_Y;
-    double* nrm = reinterpret_cast<double*>(smem + S_::OFF_NRM);  // [2][CW]
+    double2* nrm = reinterpret_cast<double2*>(smem + S_::OFF_NRM);  // [2][CW], complex128
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S_::OFF_BAR);
     uint64_t* done = full + 2;
     int4* slot = reinterpret_cast<int4*>(smem + S_::OFF_BAR + 32);  // [2] (kind, z, tile)
@@ -393,9 +393,12 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS,
                 }
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 if (!F32 && want_norm && m.kind == K2) {
-                    double q = nrm[b * S_::CW];
-                    for (int w = 1; w < S_::CW; ++w) q += nrm[b * S_::CW + w];
-                    a.red.partials[(size_t)m.z * n2 + m.tile] = make_double2(q, 0.0);
+                    KSum q{0.0, 0.0};
+                    for (int w = 0; w < S_::CW; ++w) {
+                        const double2 p = nrm[b * S_::CW + w];
+                        q.merge(p.x, p.y);
+                    }
+                    a.red.partials[(size_t)m.z * n2 + m.tile] = make_double2(q.s, q.c);
                 }
                 const int stored_x = KIND != TS_Z && m.kind == K1 ? m.z : -1;
                 // refill the buffer first: the compute warps wait for it
@@ -512,12 +515,15 @@ __global__ void __launch_bounds__(TSShape<T, N, RA, RB, P, RC>::THREADS,
                     if (F32 && want_norm) {
                         if constexpr (F32) op_norm_f32<E>(v, acc);
                     } else if (want_norm) {
-                        KSum one{0.0, 0.0};
-                        if constexpr (!F32) op_norm<T, E>(v, one);
-                        double q = one.s + one.c;
+                        KSum q{0.0, 0.0};
+                        if constexpr (!F32) op_norm<T, E>(v, q);
 #pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) q += __shfl_down_sync(0xffffffffu, q, o);
-                        if (lane == 0) nrm[b * S_::CW + warp] = q;
+                        for (int o = 16; o > 0; o >>= 1) {
+                            const double os = __shfl_down_sync(0xffffffffu, q.s, o);
+                            const double oc = __shfl_down_sync(0xffffffffu, q.c, o);
+                            q.merge(os, oc);
+                        }
+                        if (lane == 0) nrm[b * S_::CW + warp] = make_double2(q.s, q.c);
                     }
                 }
             }
