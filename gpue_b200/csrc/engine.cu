@@ -427,9 +427,11 @@ gpue_status plan_zpass(gpue_ctx* c, int prec) {
 // the rotation gauge (4 launches a step instead of 7 line passes).  An XY launch
 // has two dependent tile phases, about 9 us of latency that smaller fields,
 // which lie in L2 anyway, do not earn back.  Per step on B200, line passes and
-// tile passes: complex128 96^3 52 and 65 us, 128^3 125 and 87; with the gauge
-// complex128 96^3 85 and 85, 128^3 180 and 145, complex64 128^3 102 and 102,
-// 192^3 294 and 260.
+// tile passes: complex128 64^3 25 and 35 us, 96^3 46 and 63, 128^3 80 and 78, 160^3
+// 223 and 169; with the gauge complex128 64^3 32 and 40, 96^3 61 and 77, 128^3 115
+// and 108, complex64 96^3 49 and 59, 128^3 96 and 92 (real time 95 and 95), 160^3
+// 165 and 160 (166 and 171), 192^3 262 and 237.  The kernels below these lines are
+// not compiled.
 constexpr long kTileMin64 = 1L << 20;
 constexpr long kTileGaugeMin32 = 1L << 22;
 
@@ -439,7 +441,8 @@ gpue_status plan_xy(gpue_ctx* c, int prec) {
     const char* env = std::getenv("GPUE_XY");
     if (env && env[0] == '0') return GPUE_OK;
     if (c->dim != 3 || c->ax[0].n != c->ax[1].n || c->ax[0].n > 256) return GPUE_OK;
-    if (prec == GPUE_PREC_FP64 && c->N < kTileMin64) return GPUE_OK;
+    const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
+    if (c->N < (prec == GPUE_PREC_FP64 ? kTileMin64 : gauge ? kTileGaugeMin32 : 0)) return GPUE_OK;
     const XYKernel* k = find_xy_kernel(kprec(prec), c->ax[0].n);
     EncodeTiled enc = encode_tiled();
     if (!k || !enc) return GPUE_OK;
@@ -448,7 +451,6 @@ gpue_status plan_xy(gpue_ctx* c, int prec) {
     if (k->smem > max_smem) return GPUE_OK;
     const int n = c->ax[0].n;
     const int per = (int)(elem_size(prec) / 8), lt = 16 / per;  // 8-byte elements per value, lines per tile
-    const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
     int per_sm = 1 << 30;
     for (const void* fn : {k->fwd, gauge ? k->inv_gy : k->inv, gauge ? k->inv_gx : k->inv}) {
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem));
@@ -538,8 +540,7 @@ bool plane_ok(const gpue_ctx* c, int prec) {
     const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
     if (c->xy[prec].k) {
         if (!gauge) return true;
-        return c->xy[prec].gauge && axis_gauge_active(c, 0) && axis_gauge_active(c, 1) &&
-               (prec == GPUE_PREC_FP64 || c->N >= kTileGaugeMin32);
+        return c->xy[prec].gauge && axis_gauge_active(c, 0) && axis_gauge_active(c, 1);
     }
     return c->plane[prec].k && !gauge;
 }

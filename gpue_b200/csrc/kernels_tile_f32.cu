@@ -1,5 +1,5 @@
 // kernels_tile_f32.cu -- the complex64 TMA tile-stream XY and z passes of the
-// 3D step (tstream.cuh), per length.
+// 3D step (tstream.cuh), per length; with the gauge from 192 on (plan_xy).
 #include "tstream_tables.h"
 
 namespace gpue {
@@ -14,10 +14,10 @@ static const ZPassKernel kZPass[] = {
 };
 
 static const XYKernel kXY[] = {
-    GPUE_XY(float, 64, 4, 4, 0, 16),
-    GPUE_XY(float, 96, 4, 6, 0, 8),
-    GPUE_XY(float, 128, 4, 8, 0, 16),
-    GPUE_XY(float, 160, 4, 10, 0, 8),
+    GPUE_XY_PLAIN(float, 64, 4, 4, 0, 16),
+    GPUE_XY_PLAIN(float, 96, 4, 6, 0, 8),
+    GPUE_XY_PLAIN(float, 128, 4, 8, 0, 16),
+    GPUE_XY_PLAIN(float, 160, 4, 10, 0, 8),
     GPUE_XY(float, 192, 4, 12, 0, 16),
     GPUE_XY(float, 256, 16, 0, 0, 16),
 };

@@ -1,5 +1,5 @@
 // kernels_tile_f64.cu -- the complex128 TMA tile-stream XY and z passes of the
-// 3D step (tstream.cuh), per length.
+// 3D step (tstream.cuh), per length; the XY passes from 128 on (plan_xy).
 #include "tstream_tables.h"
 
 namespace gpue {
@@ -14,8 +14,6 @@ static const ZPassKernel kZPass[] = {
 };
 
 static const XYKernel kXY[] = {
-    GPUE_XY(double, 64, 4, 4, 0, 16),
-    GPUE_XY(double, 96, 4, 6, 0, 8),
     GPUE_XY(double, 128, 4, 8, 0, 16),
     GPUE_XY(double, 160, 4, 10, 0, 8),
     GPUE_XY(double, 192, 4, 12, 0, 16),
