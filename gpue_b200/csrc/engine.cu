@@ -2109,6 +2109,7 @@ gpue_status gpue_autotune(gpue_ctx* c, int32_t flags) {
     if (!c || (flags & ~1)) return GPUE_ERR_INVALID_ARG;
     CK(cudaSetDevice(c->device));
     CK(cudaStreamSynchronize(c->stream));
+    c->line_plan = false;  // the choice is the library's again
     return autotune_ctx(c, c->prec, (flags & 1) != 0);
 }
 

@@ -317,7 +317,8 @@ gpue_status gpue_ctx_wfc_device(gpue_ctx* ctx, void** psi, int32_t* dtype);
  * The line passes are what is tuned: they run 3D steps without tile kernels,
  * batched solves of such shapes, energy checks, and per-step fields; 2D steps
  * run on the resident steppers and 3D ones on the tile passes, which have one
- * shape per length.
+ * shape per length.  A plan set by hand (gpue_set_plan) is dropped, so a 2D
+ * context that was given one steps on the resident steppers again.
  * Setting GPUE_AUTOTUNE=1 in the environment makes gpue_ctx_create do this. */
 gpue_status gpue_autotune(gpue_ctx* ctx, int32_t flags);
 
@@ -361,7 +362,7 @@ gpue_status gpue_time_passes(gpue_ctx* ctx, int32_t gstate, int32_t nsteps, floa
  * with GPUE_ERR_INVALID_ARG when no such plan exists or the launch shape does
  * not fit the grid.  Results differ from another plan's only by round-off.  A
  * 2D context whose plan was set runs its steps as line passes with it from
- * then on, instead of the resident stepper. */
+ * then on, instead of the resident stepper, until gpue_autotune. */
 gpue_status gpue_set_plan(gpue_ctx* ctx, int32_t axis, int32_t ra, int32_t rb, int32_t rc,
                           int32_t threads_per_line, int32_t lines_per_cta);
 
