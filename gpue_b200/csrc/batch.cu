@@ -88,27 +88,32 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
            c->xy[prec].k && c->zpass[prec].k && plane_ok(c, prec);
 }
 
-// 2D solves that run on the grid-wide stepper.  Complex64 of 384^2 and 512^2, too
-// large for a cluster to step quickly alone; as many grids as the device holds
-// at once, up to 4, run side by side on lanes of their own (grid_lanes).  Per step
-// as line passes and as grids: one of 512^2 30 and 12 us, 40 of them 368 and 297
-// (one lane: 482), rotating 632 and 469; one of 384^2 42 and 11 (37 as a cluster
-// of 16), 40 of them 329 and 165 (one lane 439, clusters 222), rotating 549 and
-// 268 (729, 409).  From 768 on a grid fills the device, one after another: 8 of
-// 768^2 complex64 208 and 179, complex128 320 and 229, 8 of 1024^2 complex64 270
-// and 197, 4 of 1024^2 complex128 232 and 141.  In between the line passes are
-// faster as soon as several solves share them, 8 of 384^2 complex128 70 and 112
-// us, 8 of 640^2 198 and 208, 24 of 640^2 complex64 393 and 468, though one alone
-// is not (384^2 complex128 56 and 14); 320^2 complex64 on clusters took 29 us
-// alone and 144 as 40, rotating 53 and 267, as line passes 32, 131, 47 and 208.
-// The choice is the solve's own, never the mix's, so a result does not depend on
-// its company.
+// 2D solves that run on the grid-wide stepper. Complex64 of 512^2, and of 384^2
+// with the gauge, too large for a cluster to step quickly alone; as many grids as
+// the device holds at once, up to 4, run side by side on lanes of their own
+// (grid_lanes). Per step as line passes and as grids: one of 512^2 30 and 12 us,
+// 40 of them 368 and 297 (one lane 482), rotating 632 and 469; one rotating 384^2
+// 70 and 18 (68 as a cluster of 16), 40 of them 549 and 268 (one lane 729,
+// clusters 409). 384^2 without the gauge would take 11 as a grid and 37 as a
+// cluster (42 as line passes), 40 of them 165 and 222 (329); beside other lengths
+// clusters win, 16 solves of 128 to 512, three of them 384^2, in 12.6 and 13.5 ms.
+// From 768 on a grid fills the device, one after another: 8 of 768^2 complex64 208
+// and 179, complex128 320 and 229, 8 of 1024^2 complex64 260 and 197, 4 of 1024^2
+// complex128 232 and 141. In between the line passes are faster as soon as several
+// solves share them, 8 of 384^2 complex128 70 and 112 us, 8 of 640^2 198 and 208,
+// 24 of 640^2 complex64 393 and 468, though one alone is not (384^2 complex128 56
+// and 14); 320^2 complex64 on clusters took 29 us alone and 144 as 40, rotating 53
+// and 267, as line passes 32, 131, 47 and 208. The choice is the solve's own,
+// never the mix's, so a result does not depend on its company.
 bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
     const char* env = std::getenv("GPUE_BATCH_MEGA");
     if (env && env[0] == '0') return false;
     if (c->dim != 2 || !c->step[prec].k || c->ext || c->time_dep || c->line_plan) return false;
-    if (c->ax[0].n < 768 && (prec != GPUE_PREC_FP32 || (c->ax[0].n != 384 && c->ax[0].n != 512)))
-        return false;
+    if (c->ax[0].n < 768) {
+        const bool gauge = c->p.corotating && (axis_gauge_active(c, 0) || axis_gauge_active(c, 1));
+        if (prec != GPUE_PREC_FP32 || !(c->ax[0].n == 512 || (c->ax[0].n == 384 && gauge)))
+            return false;
+    }
     return step_ready(c, prec, gstate);
 }
 

@@ -8,6 +8,7 @@ static const ClusterKernel kTable[] = {
     GPUE_CLUSTER(float, 64, 4, 4, 0, 16),  GPUE_CLUSTER(float, 96, 4, 6, 0, 8),
     GPUE_CLUSTER(float, 128, 4, 8, 0, 16), GPUE_CLUSTER(float, 160, 4, 10, 0, 8),
     GPUE_CLUSTER(float, 192, 4, 12, 0, 16), GPUE_CLUSTER(float, 256, 8, 4, 0, 32),
+    GPUE_CLUSTER(float, 384, 4, 6, 4, 32),
 };
 
 const ClusterKernel* cluster_table_f32(int* count) {

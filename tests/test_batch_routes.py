@@ -8,7 +8,16 @@ from fake_device import fake  # noqa: F401
 LENGTHS = (16, 32, 64, 96, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024)
 # the routes' lines (batch.cu, kernels_cluster_*.cu)
 CLUSTER = {"FP32": {16, 32, 64, 96, 128, 160, 192, 256}, "FP64": {16, 32, 64, 96, 128, 192, 256}}
-GRID = {"FP32": {384, 512, 768, 1024}, "FP64": {768, 1024}}
+GRID = {"FP32": {512, 768, 1024}, "FP64": {768, 1024}}
+
+
+def routes(prec, omega):
+    """The lengths on clusters and on the grid; complex64 384^2 goes by the gauge."""
+    c, g = set(CLUSTER[prec]), set(GRID[prec])
+    if prec == "FP32":
+        (g if omega else c).add(384)
+    return c, g
+
 
 BATCH = """
 def batch(specs, gstate=0, steps=3):
@@ -35,11 +44,12 @@ def kinds(launches):
 @pytest.mark.parametrize("prec", ["FP32", "FP64"])
 @pytest.mark.parametrize("gstate,omega", [(0, 0.0), (0, 0.5), (1, 0.0), (1, 0.5)])
 def test_route_of_each_length(fake, prec, gstate, omega):  # noqa: F811
+    on_cluster, on_grid = routes(prec, omega)
     for n in LENGTHS:
         _, launches = fake(BATCH + "batch([(%d, G.PREC_%s, %g)], %d)" % (n, prec, omega, gstate))
-        if n in CLUSTER[prec]:
+        if n in on_cluster:
             assert kinds(launches) == {"k_cluster_many"}, n
-        elif n in GRID[prec]:
+        elif n in on_grid:
             assert kinds(launches) == {"k_step2d"}, n
         else:
             assert kinds(launches) <= {"k_pass_batch", "k_batch_mega"}, n
@@ -58,9 +68,9 @@ def test_equal_solves_get_equal_clusters(fake, count):  # noqa: F811
     assert size == fits[0]
 
 
-@pytest.mark.parametrize("n", [384, 512])
-def test_grids_share_lanes(fake, n):  # noqa: F811
+@pytest.mark.parametrize("n,omega", [(384, 0.3), (512, 0.0)])
+def test_grids_share_lanes(fake, n, omega):  # noqa: F811
     """One cooperative launch per solve, whatever lane it is on."""
-    _, launches = fake(BATCH + "batch([(%d, G.PREC_FP32, 0.0)] * 9)" % n)
+    _, launches = fake(BATCH + "batch([(%d, G.PREC_FP32, %g)] * 9)" % (n, omega))
     grids = [q for q in launches if "k_step2d" in q["kernel"]]
     assert len(grids) == 9 and all(q["coop"] for q in grids)

@@ -3,14 +3,14 @@ too (nothing declined for want of residency), and many alike, side by side on la
 or in clusters, end bit for bit as alone.
 
 The tests that compare those kernels with line passes (test_gpu_cluster.py,
-test_gpu_batch_grid.py) rely on it: 384^2 and 512^2 complex64 run on the grid
-stepper, 320^2 complex64 and 160^2 complex128 as line passes.
+test_gpu_batch_grid.py) rely on it: 512^2 complex64, and 384^2 with the gauge, run on
+the grid stepper, 320^2 complex64 and 160^2 complex128 as line passes.
 """
 import numpy as np
 import pytest
 
 import gpue_b200 as G
-from test_batch_routes import CLUSTER, GRID, LENGTHS
+from test_batch_routes import LENGTHS, routes
 from test_gpu_cluster import batch
 
 pytestmark = pytest.mark.gpu
@@ -24,7 +24,7 @@ def test_resident_routes_are_taken(prec, gstate, omega):
     p = getattr(G, "PREC_" + prec)
     for n in LENGTHS:
         _, stats = batch([(n, p, omega, 0)], gstate, STEPS)
-        if n in CLUSTER[prec] | GRID[prec]:
+        if n in set.union(*routes(prec, omega)):
             assert stats["kernel_launches"] == 1, n  # every step in one launch
     _, stats = batch([(640, p, omega, 0)], gstate, STEPS)  # line passes: several a step
     assert stats["kernel_launches"] > 2 * STEPS
