@@ -84,7 +84,8 @@ struct alignas(16) StepShared {
     double scale, guard;
     double target_norm, target_guard;
     int abort;
-    int pad[3];
+    unsigned more_passes;
+    unsigned long long wait_ns;
     double scratch[2 * (512 / 32)];
 };
 
@@ -122,8 +123,7 @@ __device__ __forceinline__ uint64_t step_ns() {
 }
 
 // All CTAs of the team arrive and wait; false when the wait ran out.
-__device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, uint64_t limit_ns,
-                                             StepShared* sh) {
+__device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, StepShared* sh) {
     __syncthreads();  // every thread's stores before thread 0's release
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
@@ -135,7 +135,7 @@ __device__ __forceinline__ bool step_barrier(unsigned* count, unsigned target, u
             if ((++polls & 1023u) == 0u) {
                 const uint64_t now = step_ns();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > limit_ns) {
+                else if (now - t0 > sh->wait_ns) {
                     sh->abort = 1;
                     break;
                 }
@@ -175,7 +175,7 @@ __device__ __forceinline__ unsigned slot_load(const double2* p, KSum& v) {
 // The sum of all CTAs' partials of a pass, in a fixed order, by one warp: a
 // lane reads its slots in one batch until all carry the pass's number.
 __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigned pass,
-                                            uint64_t limit_ns, StepShared* sh) {
+                                            StepShared* sh) {
     constexpr int B = 5;  // 148 CTAs in one batch
     const int lane = threadIdx.x & 31;
     KSum r{0.0, 0.0};
@@ -194,7 +194,7 @@ __device__ __forceinline__ double slots_sum(const double2* slots, int n, unsigne
             if ((++polls & 1023u) == 0u) {
                 const uint64_t now = step_ns();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > limit_ns) {
+                else if (now - t0 > sh->wait_ns) {
                     sh->abort = 1;
                     break;
                 }
@@ -265,6 +265,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
     }
     if (tid == 0) {
         sh->abort = 0;
+        sh->more_passes = s.more_passes;
+        sh->wait_ns = s.wait_ns;
         sh->scale = *s.scal_norm;
         sh->guard = *s.scal_guard;
         sh->target_norm = *s.target_norm;
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     cx<T> v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = cx<T>{(T)0, (T)0};
-    unsigned target = 0;
+    unsigned target = s.more_ctas;
     StepPass sp = s.seq[0];
     for (int k = 0; k < s.nseq; ++k) {
         const bool colpass = sp.flags & SP_COL;
@@ -450,14 +452,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
         }
         if (flags & SP_SYNC) {
             target += (unsigned)ncta;
-            if (!step_barrier(s.sync, target + s.more_ctas, s.wait_ns, sh)) break;
+            if (!step_barrier(s.sync, target, sh)) break;
         }
         if (flags & (SP_NORM | SP_GUARD)) {
             // (a CTA overwrites its slot at the next norm only, and a barrier
             // that every reader of this one has reached lies between)
             if (tid < 32) {
                 const double sum =
-                    slots_sum(s.slots, ncta, (unsigned)k + 1 + s.more_passes, s.wait_ns, sh);
+                    slots_sum(s.slots, ncta, (unsigned)k + 1 + sh->more_passes, sh);
                 if (tid == 0) {
                     if (flags & SP_NORM) sh->scale = sqrt(sh->target_norm / sum);
                     else sh->guard = sqrt(sh->target_guard / sum);
