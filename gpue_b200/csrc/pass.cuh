@@ -802,7 +802,7 @@ __device__ __forceinline__ KSum pass_tiles(const PassArgs& a, long t0, long tste
                     const double ang1 = a.gauge_coef * a.pos[src][sidx] * a.gauge_dt * a.dmom;
                     // (one branch per time kind, so that only its own constants are
                     // held: with both the 640 complex64 column pass spilled 524 bytes
-                    // instead of 364, 8 batched 640^2 151 us per step instead of 144)
+                    // instead of 364, 8 batched 640^2 150 us per step instead of 146)
                     if (a.gstate == 0)
                         op_gauge<T, L>(v, gauge_consts<L>(t, ang1, 0, a.gscale), 0);
                     else

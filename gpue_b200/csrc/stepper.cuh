@@ -27,14 +27,15 @@
 // What bounds it, and the shapes.  A pass is latency: at 256^2 complex128 it
 // takes about 780 cycles to load, 2200 to transform twice, 1900 in the barrier
 // and 1800 per norm; at 1024^2 complex64 the SMs with most lines issue 85 % of
-// their cycles.  So the lines are dealt out as one CTA per SM (C a
-// divisor of n, at least n/148) where a line has at most 32 threads; lines of 64 threads run as
+// their cycles.  So the lines are dealt out as one CTA per SM (C a divisor of n,
+// at least n/148) where a line has at most 32 threads; lines of 64 threads run as
 // several smaller CTAs per SM, whose column barriers then stop 2 to 8 warps
 // instead of all (1024^2 complex64: 42 us per step as 256 CTAs of 4 lines, 48
-// as 147 CTAs of 7).  Time per step on B200, before as line passes and now:
-// complex128 64^2 11.6 -> 7.1 us, 256^2 15.3 -> 9.7, 320^2 (real time) 27.4 ->
-// 13.8, 384^2 rotating 34.2 -> 22.2, 1024^2 rotating 67.8 -> 66.0; complex64
-// 256^2 13.3 -> 8.2, 640^2 36 -> 19.5, 1024^2 rotating 47.6 -> 42.7.
+// with 7 lines and 147 CTAs).  Time per step on B200, as line passes before this
+// kernel and now: complex128 128^2 15.3 -> 8.5 us, 256^2 15.7 -> 9.0, 320^2 (real
+// time) 27.4 -> 12.2, 384^2 rotating 34.2 -> 21.4, 768^2 42.8 -> 27.9, 1024^2
+// rotating 68.2 -> 59.4; complex64 256^2 13.3 -> 8.1, 640^2 35.8 -> 19.7, 768^2
+// 31.3 -> 22.2, 1024^2 rotating 47.6 -> 39.7.
 #pragma once
 
 #include <type_traits>

@@ -23,23 +23,23 @@
 // it.  The compute warps only wait for full[b].
 //
 // XY ordering (for y then x exchange the two).  Tickets follow: the x-tiles of
-// plane g, then the y-tiles of plane g - LAG, for g = 0, 1, ...  A y-tile of plane z may load only after
-// all x-tiles of plane z are stored (a per-plane count, raised with release
-// semantics by each x-tile's producer once its store is complete, and read
-// with acquire semantics); by then the plane is normally still in L2, so the
-// field crosses HBM once in and once out.  The producer counts an x-tile as
-// soon as its store completes, after it has refilled the buffer (the compute
-// warps are busy with the other buffer meanwhile).  LAG (64 planes by
-// default: shorter lags leave y-tiles waiting, longer ones overflow L2) is
-// set per context.  A producer whose next y-tile's plane is not ready only
-// marks the buffer pending, and waits (bounded) for it when that buffer's
-// turn comes, when every tile it held with a smaller ticket is stored and
-// counted.  A waited-for x-tile therefore always has a smaller ticket
-// than the wait, and a CTA holding one either is not waiting or waits for a
-// still smaller ticket: no cycle, and the smallest waiting ticket's x-tiles
-// are all held by CTAs that finish them.  Every wait is bounded; one that
-// gives up sets *err (the host reports GPUE_ERR_TIMEOUT), and the kernel then
-// drains its copies in flight before it returns.
+// plane g, then the y-tiles of plane g - LAG, for g = 0, 1, ...  A y-tile of
+// plane z may load only after all x-tiles of plane z are stored (a per-plane
+// count, raised with release semantics by each x-tile's producer once its store
+// is complete, and read with acquire semantics); by then the plane is normally
+// still in L2, so the field crosses HBM once in and once out.  The producer
+// counts an x-tile as soon as its store completes, after it has refilled the
+// buffer (the compute warps are busy with the other buffer meanwhile).  LAG
+// (plan_xy: by plane size; shorter lags leave y-tiles waiting, longer ones
+// overflow L2) is set per context.  A producer whose next y-tile's plane is not
+// ready only marks the buffer pending, and waits (bounded) for it when that
+// buffer's turn comes, when every tile it held with a smaller ticket is stored
+// and counted.  A waited-for x-tile therefore always has a smaller ticket than
+// the wait, and a CTA holding one either is not waiting or waits for a still
+// smaller ticket: no cycle, and the smallest waiting ticket's x-tiles are all
+// held by CTAs that finish them.  Every wait is bounded; one that gives up sets
+// *err (the host reports GPUE_ERR_TIMEOUT), and the kernel then drains its
+// copies in flight before it returns.
 //
 // The counters reset themselves: the last CTA to finish clears the ticket,
 // the per-plane counts and its own finish count, so consecutive launches need
@@ -56,8 +56,9 @@
 // cycle).  Complex128: shared memory, so its 256-point plan is the one with a
 // single exchange (16 x 16, 16 values a thread: 433 us per 256^3 step; 8 x 4 x 8
 // with twice the warps 520).  The z pass then moves 4.9 TB/s, the XY passes 3.2.
-// Per step of 256^3 complex128, five line passes and these three: 809 -> 426 us;
-// 128^3 125 -> 87; with the gauge 256^3 1170 -> 780, complex64 704 -> 506.
+// Per step of 256^3 complex128, five line passes and these three: 808 -> 429 us;
+// 192^3 404 -> 254; with the gauge 256^3 1197 -> 703, complex64 696 -> 472.  (The
+// line passes have become faster since: 128^3 complex128 124, now 80, and 78 here.)
 //
 // The norm in complex128: every warp leaves its compensated FP64 sum of a tile
 // with the producer, which adds the warps' in order into the tile's partial; the
