@@ -24,10 +24,12 @@
 // threads at 64 registers were no faster: 256^2 45 -> 50 us); the rest is the
 // column groups' barriers and remote loads.  Batched complex64 solves on B200,
 // point-steps/s of the multi-size line-pass kernel and here: 128 of 128^2 2.0e10
-// -> 5.6e10, 64 of 192^2 1.75e10 -> 5.4e10, 32 of 256^2 1.9e10 -> 4.7e10, 16 of
-// 384^2 1.4e10 -> 2.2e10 (7 clusters of 16 at a time); complex128 32 of 128^2
-// 1.4e10 -> 3.1e10.  A lone solve gets 16 SMs at most: complex128 256^2 39 -> 19 us per
-// step, but complex64 512^2 30 -> 55, so that one runs on the grid (batch.cu).
+// -> 5.4e10, 64 of 192^2 1.75e10 -> 5.3e10, 32 of 256^2 1.9e10 -> 4.6e10, 16 of
+// 384^2 1.4e10 -> 2.1e10 (7 clusters of 16 at a time); complex128 32 of 128^2
+// 1.35e10 -> 3.0e10.  One case is slower: 8 of 256^2 complex64, one more than fit as
+// 16 CTAs, take 25 us per step in real time (23) and 48 rotating (43).  A lone solve
+// gets 16 SMs at most: complex128 256^2 39 -> 20 us per step, but complex64 512^2
+// 30 -> 55, so that one runs on the grid (batch.cu).
 //
 // Shared memory per CTA: the rows at a padded stride, which double as the
 // exchange buffer of their own transforms; an exchange buffer for the columns
@@ -66,7 +68,7 @@ struct ClusterShape {
     using L = LineFFT<T, N, RA, RB, P, RC>;
     static constexpr int E = L::E;
     // (256^2 complex128: 16 lines of 16 threads, so that clusters of 8 hold it
-    // with one exchange per transform: 8 solves 30.6 us per step; 8 4 8 with 512
+    // with one exchange per transform: 8 solves 31.9 us per step; 8 4 8 with 512
     // threads needs clusters of 16, 40.8)
     static constexpr int MOST = sizeof(T) == 8 && N == 256 ? 256 : kClusterThreads;
     static constexpr int THREADS = N * P < MOST ? N * P : MOST;
