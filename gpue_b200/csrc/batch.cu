@@ -103,7 +103,7 @@ bool tile_eligible(const gpue_ctx* c, int prec) {
 // solves share them, 8 of 384^2 complex128 70 and 112 us, 8 of 640^2 198 and 208,
 // 24 of 640^2 complex64 393 and 468, though one alone is not (384^2 complex128 56
 // and 14); 320^2 complex64 on clusters took 29 us alone and 144 as 40, rotating 53
-// and 267, as line passes 32, 131, 47 and 208. The choice is the solve's own,
+// and 267, as line passes 31, 128, 47 and 204. The choice is the solve's own,
 // never the mix's, so a result does not depend on its company.
 bool grid_eligible(gpue_ctx* c, int prec, int gstate) {
     const char* env = std::getenv("GPUE_BATCH_MEGA");

@@ -26,10 +26,10 @@
 // point-steps/s of the multi-size line-pass kernel and here: 128 of 128^2 2.0e10
 // -> 5.4e10, 64 of 192^2 1.75e10 -> 5.3e10, 32 of 256^2 1.9e10 -> 4.6e10, 16 of
 // 384^2 1.4e10 -> 2.1e10 (7 clusters of 16 at a time); complex128 32 of 128^2
-// 1.35e10 -> 3.0e10.  One case is slower: 8 of 256^2 complex64, one more than fit as
-// 16 CTAs, take 25 us per step in real time (23) and 48 rotating (43).  A lone solve
-// gets 16 SMs at most: complex128 256^2 39 -> 20 us per step, but complex64 512^2
-// 30 -> 55, so that one runs on the grid (batch.cu).
+// 1.35e10 -> 3.0e10.  Slower: 8 complex64 solves, one more than fit as 16 CTAs,
+// of 256^2 25 us per step in real time (23) and 48 rotating (42), of 384^2 72
+// (67).  A lone solve gets 16 SMs at most: complex128 256^2 39 -> 20 us per
+// step, but complex64 512^2 30 -> 55, so that one runs on the grid (batch.cu).
 //
 // Shared memory per CTA: the rows at a padded stride, which double as the
 // exchange buffer of their own transforms; an exchange buffer for the columns
